@@ -614,10 +614,29 @@ public:
 
     // ---- z-marching launches ----
     static constexpr int TX = 32, TY = 8;
-    int zchunk(int gxy, int minlen) const {
-        int nch = (4 * 148 * 8 + gxy - 1) / gxy;
-        nch = std::max(1, std::min(nch, mz / minlen));
-        return (mz + nch - 1) / nch;
+    // CTAs per SM of a kernel, asked once per context (a member: several builds of the library may
+    // share a process, and a function-local static of a template would be shared between them)
+    std::vector<std::pair<const void*, int>> resident_of;
+    int resident(const void* fn, int threads, size_t smem) {
+        for (const auto& r : resident_of)
+            if (r.first == fn) return r.second;
+        int n = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, threads, smem) != cudaSuccess || n < 1) n = 1;
+        resident_of.push_back({fn, n});
+        return n;
+    }
+    // z planes per CTA of a z-marching launch over gxy tiles: 16 or more planes where that gives the
+    // GPU its fill of CTAs (longer marches, one wave of them, measured 5-10 % slower on 512x256x256:
+    // the CTAs of a wave then spread over all z), and where it does not, as many planes as make one
+    // wave of all CTAs, two at least (a CTA's march is a serial chain of plane steps: on 64x32x64
+    // 16 planes a CTA left 20 CTAs of 148 SMs busy and took 1.47 ms a step in FP64, 1.33 in FP32;
+    // two planes 0.70 and 0.58, three 0.78 and 0.61)
+    int zchunk(int gxy, const void* fn, int threads, size_t smem) {
+        const double slots = 148.0 * resident(fn, threads, smem);
+        const int nch = std::max(1, std::min((4 * 148 * 8 + gxy - 1) / gxy, mz / 16));
+        if ((double)gxy * nch > 1.5 * slots) return (mz + nch - 1) / nch;
+        const int one = std::max(1, (int)(slots / gxy));
+        return std::max(2, (mz + one - 1) / one);
     }
     // radius-2 ring kernels (k_zst2): 32 x 8 columns per CTA
     static constexpr int ZTX = 32;
@@ -677,7 +696,14 @@ public:
     void zp(const char* tag, double bytes, const SrcFields<T, NF>& src, const Epi& epi) {
         using Z = ZVc<NF>;
         dim3 gg((mx + Z::TX - 1) / Z::TX, (my + Z::TY - 1) / Z::TY, 1);
-        int ch = zchunk(gg.x * gg.y, 16);
+        int ch = 0;
+        if constexpr (zp_tma<NF>()) {
+#ifndef DASHA_NO_TMA
+            ch = zchunk(gg.x * gg.y, (const void*)zpv_tma_fn<NF, KINDS, Epi, MODE>(), 32 * ZC<NF>::TYH, Z::smem_tma());
+#endif
+        } else {
+            ch = zchunk(gg.x * gg.y, (const void*)zpv_fn<NF, KINDS, Epi, MODE>(), 32 * ZC<NF>::TYH, Z::smem());
+        }
         gg.z = (mz + ch - 1) / ch;
 #ifndef DASHA_NO_TMA
         if constexpr (zp_tma<NF>()) {
@@ -725,7 +751,7 @@ public:
     void zp2(const char* tag, double bytes, const SrcFields<T, NF>& src, const Epi& epi) {
         using Z = ZV2c<NF>;
         dim3 gg((mx + Z::TX - 1) / Z::TX, (my + ZC2<NF>::TY - 1) / ZC2<NF>::TY, 1);
-        int ch = zchunk(gg.x * gg.y, 16);
+        int ch = zchunk(gg.x * gg.y, (const void*)zpv2_fn<NF, KINDS, Epi>(), 32 * Z::NW, Z::smem());
         gg.z = (mz + ch - 1) / ch;
         DASHA_LAUNCH(tag, bytes, (zpv2_fn<NF, KINDS, Epi>()<<<gg, 32 * Z::NW, Z::smem(), st>>>(g, src, epi, ch)));
     }
@@ -739,7 +765,7 @@ public:
     template <int SIGN>
     void zcurl(const char* tag, const SrcFields<T, 3>& src, F3<T> out) {
         dim3 gg((mx + ZC3c::TX - 1) / ZC3c::TX, (my + 7) / 8, 1);
-        int ch = zchunk(gg.x * gg.y, 16);
+        int ch = zchunk(gg.x * gg.y, (const void*)k_zcurl<T, ZVX, 8, 2, SIGN>, 256, ZC3c::smem());
         gg.z = (mz + ch - 1) / ch;
         DASHA_LAUNCH(tag, 6.0 * N * sizeof(T), (k_zcurl<T, ZVX, 8, 2, SIGN><<<gg, 256, ZC3c::smem(), st>>>(g, src, out, ch)));
     }
@@ -973,7 +999,7 @@ public:
             eh.j1 = curF[0]; eh.j2 = curF[1]; eh.j3 = curF[2];
             for (int q = 0; q < 3; ++q) { eh.e[q] = E[0][q]; eh.h[q] = Hh[0][q]; }
             dim3 ge((mx + ZEHc::TX - 1) / ZEHc::TX, (my + 7) / 8, 1);
-            int che = zchunk(ge.x * ge.y, 16);
+            int che = zchunk(ge.x * ge.y, (const void*)k_zeh<T, ZVX, 8, 2>, 256, ZEHc::smem());
             ge.z = (mz + che - 1) / che;
             DASHA_LAUNCH("k_efield_hall", 17.0 * N * sizeof(T), (k_zeh<T, ZVX, 8, 2><<<ge, 256, ZEHc::smem(), st>>>(g, eh, che)));
             hx(Hh[0], 3);
@@ -997,16 +1023,17 @@ public:
             Ef = passes3<0u>("k_zpv_E", E[0], E[1], 4, true);
         }
         // right-hand side: hydro part (xdif 0..3, 7) and induction (xdif 4..6)
-        dim3 gg(mx / ZTX, (my + 7) / 8, 1);
-        int ch = zchunk(gg.x * gg.y, 32);
-        gg.z = (mz + ch - 1) / ch;
         if (!g.viscos && !g.diffu) {   // register-blocked fast path (no viscosity, no diffusion)
             HydroIO<T> hio;
             hio.drho = xs[0]; hio.m1 = xs[1]; hio.m2 = xs[2]; hio.m3 = xs[3]; hio.dp = xs[7];
             hio.j1 = curF[0]; hio.j2 = curF[1]; hio.j3 = curF[2]; hio.b1 = xs[4]; hio.b2 = xs[5]; hio.b3 = xs[6];
             hio.out[0] = K[0]; hio.out[1] = K[1]; hio.out[2] = K[2]; hio.out[3] = K[3]; hio.out[4] = K[7];
             dim3 gh((mx + ZHc::TX - 1) / ZHc::TX, (my + ZH_TY - 1) / ZH_TY, 1);
-            int chh = zchunk(gh.x * gh.y, 16);
+#ifndef DASHA_NO_TMA
+            int chh = zchunk(gh.x * gh.y, (const void*)k_zhydro_tma<T, ZH_VX, ZH_TY, 1, ZH_MINB>, 32 * ZH_TY, ZHc::smem_tma());
+#else
+            int chh = zchunk(gh.x * gh.y, (const void*)k_zhydro<T, ZH_VX, ZH_TY, 1, ZH_MINB>, 32 * ZH_TY, ZHc::smem());
+#endif
             gh.z = (mz + chh - 1) / chh;
 #ifndef DASHA_NO_TMA
             ZhMaps maps;
@@ -1018,6 +1045,9 @@ public:
                          (k_zhydro<T, ZH_VX, ZH_TY, 1, ZH_MINB><<<gh, 32 * ZH_TY, ZHc::smem(), st>>>(g, hio, chh)));
 #endif
         } else {
+        dim3 gg(mx / ZTX, (my + 7) / 8, 1);
+        int ch = zchunk(gg.x * gg.y, (const void*)k_zst2<T, 5, ZTX, 8, HMINB, OpHydro<T>>, ZTX * 8, ZS2<T, 5, ZTX, 8>::smem(true));
+        gg.z = (mz + ch - 1) / ch;
         SrcFields<T, 5> sh;
         sh.f[0] = xs[0]; sh.f[1] = xs[1]; sh.f[2] = xs[2]; sh.f[3] = xs[3]; sh.f[4] = xs[7];
         OpHydro<T> oh;
