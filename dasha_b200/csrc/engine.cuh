@@ -297,6 +297,7 @@ public:
             *w2[d][0] = t + off[d][8]; *w2[d][1] = t + off[d][9];
         }
         g.cbx = t + offcb;
+        g.cr = E[1][0];
         g.xc = t + off[0][10]; g.yc = t + off[1][10]; g.zc = t + off[2][10];
         g.eta = T(p.eta); g.di = T(p.di); g.gamma = T(p.gamma); g.mu = T(p.mu); g.drho = T(p.drho); g.dp = T(p.dp);
         g.hall = p.hall; g.viscos = p.viscos && p.mu != 0.0; g.diffu = p.diffu && (p.drho != 0.0 || p.dp != 0.0);
@@ -354,6 +355,7 @@ public:
         blk = dim3(std::min(128, ((mx + 31) / 32) * 32));
         grd = dim3((mx + blk.x - 1) / blk.x, my, mz);
         DASHA_CK(zs_attr());
+        if (!KAHAN) k_radial_field<T><<<grd, blk, 0, st>>>(g, E[1][0]);
         DASHA_CK(cudaStreamSynchronize(st));
         return Status::ok();
     }
@@ -989,8 +991,7 @@ public:
     void launch_rhs_raw(T* const* xs) {
         NvtxRange range("right");
         launch_current(xs);
-        T** cother = curF == cur[0] ? cur[1] : cur[0];
-        (void)cother;
+        T** cother = curF == cur[0] ? cur[1] : cur[0];   // free until the next current: the E chain's second buffer
         // E0 = -v x B + eta J at every node, then avrgE's 4 passes (t3dsdsc.f:1367-1389)
         if (P.hall) {   // E0 and the Hall field in one z-march over the state
             EHIO<T> eh;
@@ -1011,8 +1012,8 @@ public:
             // avrgh passes 1-4, avrgE passes 1-3, then one 6-field launch: the 4th E pass and the
             // 5th Hall pass, summed into E (the two chains are independent until that sum)
             T** h = passes3<KIND_H>("k_zpv_H", Hh[0], Hh[1], 4, true);
-            T** e3 = passes3<0u>("k_zpv_E", E[0], E[1], 3, true);
-            T** eo = e3 == E[0] ? E[1] : E[0];
+            T** e3 = passes3<0u>("k_zpv_E", E[0], cother, 3, true);
+            T** eo = e3 == E[0] ? cother : E[0];
             SrcFields<T, 6> se;
             VSum<T, 3, ZVX> es;
             for (int q = 0; q < 3; ++q) { se.f[q] = e3[q]; se.f[3 + q] = h[q]; es.f[q] = eo[q]; }
@@ -1020,7 +1021,7 @@ public:
             Ef = eo;
             hx(Ef, 3);
         } else {
-            Ef = passes3<0u>("k_zpv_E", E[0], E[1], 4, true);
+            Ef = passes3<0u>("k_zpv_E", E[0], cother, 4, true);
         }
         // right-hand side: hydro part (xdif 0..3, 7) and induction (xdif 4..6)
         if (!g.viscos && !g.diffu) {   // register-blocked fast path (no viscosity, no diffusion)

@@ -63,6 +63,16 @@ __device__ __forceinline__ float radial_coef_fast(float r2) {
 }
 __device__ __forceinline__ double radial_coef_fast(double r2) { return radial_coef(sqrt(r2)); }
 
+// the radial coefficient at every node (FP64 contexts, once at creation)
+template <class T>
+__global__ void k_radial_field(Geo<T> g, T* cr) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= g.mx) return;
+    const int j = blockIdx.y, k = blockIdx.z;
+    cr[(long)i + (long)j * g.sy + (long)k * g.sz] =
+        radial_coef_fast(g.xc[i] * g.xc[i] + g.yc[j] * g.yc[j] + g.zc[k] * g.zc[k]);
+}
+
 // KINDS (2 bits per field): does any of the first nf fields use the radial coefficient
 __host__ __device__ constexpr bool any_kind0(unsigned kinds, int nf) {
     for (int f = 0; f < nf; ++f)

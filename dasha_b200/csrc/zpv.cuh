@@ -22,7 +22,11 @@
 // keep the cp.async copies.  The compute is the same code in both kernels; the engine picks one
 // per launch.
 //
-// KINDS: 2 bits per output field, 0 radial coefficient, 1 constant 1/8, 2 x-profile cbx.
+// KINDS: 2 bits per output field, 0 radial coefficient, 1 constant 1/8, 2 x-profile cbx.  The
+// radial coefficient is evaluated per node in FP32 (__expf) and read from the context's field
+// g.cr in FP64, where a square root and a tanh per node and pass set the pace: with the field and its
+// L2 fetch a 3-field pass takes 98 us instead of 109 on 256x128x256 (one more 8-byte read per
+// node) and 9 us instead of 10 on 64x32x64.
 // MODE 0 writes the smoothed fields through the epilogue.  MODES 1 and 2 are the two passes of
 // avrgtt on a compensated FP32 state (x, comp) whose value is x - comp: MODE 1 reads x in
 // fields 0..NF/2-1 and comp in the rest and writes the first pass's increment d of x - comp;
@@ -57,6 +61,9 @@ struct VIO<float, 2> {
         *reinterpret_cast<float2*>(p) = make_float2(v[0], v[1]);
     }
 };
+
+// the 32-byte sector of p into L2
+__device__ __forceinline__ void l2_fetch(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 // ---- epilogues: pre(i, p) loads the operands of the VX nodes starting at i (issued before
 // the plane's barrier so that the loads overlap it), store(i, v, p) writes them; wall(i, v)
@@ -234,6 +241,7 @@ __device__ __forceinline__ void zpv_body(const Geo<T>& g, const SrcFields<T, NF>
                   CH = Z::CH;
     constexpr int NT = 32 * TYH;
     constexpr int NO = MODE == 1 ? NF / 2 : NF;       // output fields
+    constexpr bool CRF = sizeof(T) == 8 && any_kind0(KINDS, NO);   // the radial coefficient is read, not evaluated
     static_assert(MODE != 1 || NF % 2 == 0, "MODE 1 reads (x, comp) field pairs");
     constexpr int NVEC = Z::NR * CH;                  // 16-byte copies per field-plane
     constexpr int NHAL = 2 * TY;                      // halo-column element copies
@@ -348,10 +356,17 @@ __device__ __forceinline__ void zpv_body(const Geo<T>& g, const SrcFields<T, NF>
         issue(c + 1 + D);
         const T wpz = g.wpz[c], wmz = g.wmz[c], wsz = wpz + wmz, zz2 = g.zc[c] * g.zc[c];
         typename Epi::Pre pre[RY];
+        T cr[RY][VX];
 #pragma unroll
         for (int u = 0; u < RY; ++u)
-            if (xon && gj[u] < g.my && DASHA_SPAN((long)gi + (long)gj[u] * g.sy + (long)c * g.sz, VX, g.sz * (long)g.mz, BS_ZPV_STORE))
-                epi.pre((long)gi + (long)gj[u] * g.sy + (long)c * g.sz, pre[u]);
+            if (xon && gj[u] < g.my && DASHA_SPAN((long)gi + (long)gj[u] * g.sy + (long)c * g.sz, VX, g.sz * (long)g.mz, BS_ZPV_STORE)) {
+                const long i = (long)gi + (long)gj[u] * g.sy + (long)c * g.sz;
+                epi.pre(i, pre[u]);
+                if constexpr (CRF) {
+                    IO::ld(g.cr + i, cr[u]);
+                    l2_fetch(g.cr + i + g.sz);        // plane c+1 <= mz-2
+                }
+            }
 #ifndef DASHA_NO_TMA
         if (tma) {
             // planes c-1 .. c+1 on the first step, then c+1
@@ -406,9 +421,10 @@ __device__ __forceinline__ void zpv_body(const Geo<T>& g, const SrcFields<T, NF>
                 xle[f] = pc[f * SP + base + u * RS - 1];
                 xri[f] = pc[f * SP + base + u * RS + VX];
             }
-            T cr[VX];
+            if constexpr (!CRF) {
 #pragma unroll
-            for (int e = 0; e < VX; ++e) cr[e] = any_kind0(KINDS, NO) ? radial_coef_fast(xx2[e] + yy2[u] + zz2) : T(0);
+                for (int e = 0; e < VX; ++e) cr[u][e] = any_kind0(KINDS, NO) ? radial_coef_fast(xx2[e] + yy2[u] + zz2) : T(0);
+            }
             // neighbour f, e in direction: x-, x+, y-, y+ (own strip from registers)
             auto nxm = [&](int f, int e) { return e > 0 ? q0[u][f][e > 0 ? e - 1 : 0] : xle[f]; };
             auto nxp = [&](int f, int e) { return e < VX - 1 ? q0[u][f][e < VX - 1 ? e + 1 : e] : xri[f]; };
@@ -431,7 +447,7 @@ __device__ __forceinline__ void zpv_body(const Geo<T>& g, const SrcFields<T, NF>
                         const T tym = (x0v - nym(f, e)) - (k0v - nym(f + NO, e));
                         const T tzp = (qp[u][f][e] - x0v) - (qp[u][f + NO][e] - k0v);
                         const T tzm = (x0v - qm[u][f][e]) - (k0v - qm[u][f + NO][e]);
-                        const T coef = kind == 0u ? cr[e] : (kind == 1u ? T(0.125) : cbx[e]);
+                        const T coef = kind == 0u ? cr[u][e] : (kind == 1u ? T(0.125) : cbx[e]);
                         val[f][e] = coef * (txp * wpx[e] - txm * wmx[e] + typ * wpy[u] - tym * wmy[u] + tzp * wpz - tzm * wmz);
                     }
                 }
@@ -484,7 +500,7 @@ __device__ __forceinline__ void zpv_body(const Geo<T>& g, const SrcFields<T, NF>
                         sn = __ffma2_rn(Wmy, make_float2(nym(f, 0), nym(f, 1)), sn);
                         sn = __ffma2_rn(Wpz, make_float2(qp[u][f][0], qp[u][f][1]), sn);
                         sn = __ffma2_rn(Wmz, make_float2(qm[u][f][0], qm[u][f][1]), sn);
-                        const float2 cf = kind == 0u ? make_float2(cr[0], cr[1])
+                        const float2 cf = kind == 0u ? make_float2(cr[u][0], cr[u][1])
                                                      : (kind == 1u ? make_float2(0.125f, 0.125f) : make_float2(cbx[0], cbx[1]));
                         const float2 a = __ffma2_rn(make_float2(-cf.x, -cf.y), Ws, one);
                         const float2 r = __ffma2_rn(cf, sn, __fmul2_rn(a, v0));
@@ -504,7 +520,7 @@ __device__ __forceinline__ void zpv_body(const Geo<T>& g, const SrcFields<T, NF>
                             sn = fma(wmy[u], nym(f, e), sn);
                             sn = fma(wpz, qp[u][f][e], sn);
                             sn = fma(wmz, qm[u][f][e], sn);
-                            const T coef = kind == 0u ? cr[e] : (kind == 1u ? T(0.125) : cbx[e]);
+                            const T coef = kind == 0u ? cr[u][e] : (kind == 1u ? T(0.125) : cbx[e]);
                             const T a = fma(-coef, wsum[e], MODE == 2 ? T(2) : T(1));
                             val[f][e] = fma(coef, sn, a * v0);
                         }
