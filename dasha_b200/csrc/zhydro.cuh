@@ -189,6 +189,11 @@ __device__ __forceinline__ void zhydro_body(const Geo<T>& g, const HydroIO<T>& i
             const long q = col + (long)c * g.sz;
             IO::ld(io.j1 + q, j1); IO::ld(io.j2 + q, j2); IO::ld(io.j3 + q, j3);
             IO::ld(io.b1 + q, b1); IO::ld(io.b2 + q, b2); IO::ld(io.b3 + q, b3);
+            if (c < cB) {   // the next plane's into L2 (FP64 256x128x256: 354 -> 331 us; FP32 512x256x256: 746 -> 728 us)
+                const long f = q + g.sz;
+                l2_fetch(io.j1 + f); l2_fetch(io.j2 + f); l2_fetch(io.j3 + f);
+                l2_fetch(io.b1 + f); l2_fetch(io.b2 + f); l2_fetch(io.b3 + f);
+            }
         }
         const T az = g.a1z[c], bz = g.b1z[c], cz = g.c1z[c], dz = g.d1z[c];
 #ifndef DASHA_NO_TMA

@@ -66,13 +66,18 @@ struct VIO<float, 2> {
 __device__ __forceinline__ void l2_fetch(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 // ---- epilogues: pre(i, p) loads the operands of the VX nodes starting at i (issued before
-// the plane's barrier so that the loads overlap it), store(i, v, p) writes them; wall(i, v)
-// writes a wall row (no prefetch) ----
+// the plane's barrier so that the loads overlap it), fetch(i) brings them into L2 one plane ahead,
+// store(i, v, p) writes them; wall(i, v) writes a wall row (no prefetch).  The fetch costs one
+// instruction a row and operand and no register, and leaves an L2 latency of the DRAM latency each
+// plane step waited for: RK update passes 329 -> 274 us (256x128x256 FP64, mean of the stages), 541 -> 487 us
+// (512x256x256 FP32).  The same operands kept in registers a plane ahead cost a CTA per SM and
+// were slower. ----
 template <class T, int NF, int VX>
 struct VStore {
     T* f[NF];
     struct Pre {};
     __device__ __forceinline__ void pre(long, Pre&) const {}
+    __device__ __forceinline__ void fetch(long) const {}
     __device__ __forceinline__ void store(long i, const T (&v)[NF][VX], const Pre&) const { wall(i, v); }
     __device__ __forceinline__ void wall(long i, const T (&v)[NF][VX]) const {
 #pragma unroll
@@ -85,6 +90,7 @@ struct VAcc {   // f = a + v  (a may alias f: each node is read and written by o
     T* f[NF];
     const T* a[NF];
     struct Pre { T a[NF][VX]; };
+    __device__ __forceinline__ void fetch(long) const {}
     __device__ __forceinline__ void pre(long i, Pre& p) const {
 #pragma unroll
         for (int q = 0; q < NF; ++q) VIO<T, VX>::ld(a[q] + i, p.a[q]);
@@ -112,6 +118,7 @@ struct VSum {
     T* f[NO];
     struct Pre {};
     __device__ __forceinline__ void pre(long, Pre&) const {}
+    __device__ __forceinline__ void fetch(long) const {}
     __device__ __forceinline__ void store(long i, const T (&v)[2 * NO][VX], const Pre&) const { wall(i, v); }
     __device__ __forceinline__ void wall(long i, const T (&v)[2 * NO][VX]) const {
 #pragma unroll
@@ -136,6 +143,15 @@ struct VRK {
     int stage;
     double dt;
     struct Pre { T b[NF][VX], a[NF][VX], k[NF][VX]; };
+    // the operands of pre(i, .) into L2
+    __device__ __forceinline__ void fetch(long i) const {
+#pragma unroll
+        for (int q = 0; q < NF; ++q) {
+            if (!(stage == 4 && !KAHAN)) l2_fetch(base[q] + i);
+            if (stage != 1) l2_fetch(acc[q] + i);
+            if (KAHAN && stage == 4) l2_fetch(comp[q] + i);
+        }
+    }
     __device__ __forceinline__ void pre(long i, Pre& p) const {
 #pragma unroll
         for (int q = 0; q < NF; ++q) {
@@ -191,6 +207,10 @@ struct VKF {
     T* x[NF];
     T* comp[NF];
     struct Pre { T x[NF][VX], k[NF][VX]; };
+    __device__ __forceinline__ void fetch(long i) const {
+#pragma unroll
+        for (int q = 0; q < NF; ++q) { l2_fetch(x[q] + i); l2_fetch(comp[q] + i); }
+    }
     __device__ __forceinline__ void pre(long i, Pre& p) const {
 #pragma unroll
         for (int q = 0; q < NF; ++q) { VIO<T, VX>::ld(x[q] + i, p.x[q]); VIO<T, VX>::ld(comp[q] + i, p.k[q]); }
@@ -362,6 +382,7 @@ __device__ __forceinline__ void zpv_body(const Geo<T>& g, const SrcFields<T, NF>
             if (xon && gj[u] < g.my && DASHA_SPAN((long)gi + (long)gj[u] * g.sy + (long)c * g.sz, VX, g.sz * (long)g.mz, BS_ZPV_STORE)) {
                 const long i = (long)gi + (long)gj[u] * g.sy + (long)c * g.sz;
                 epi.pre(i, pre[u]);
+                if (c < cB) epi.fetch(i + g.sz);
                 if constexpr (CRF) {
                     IO::ld(g.cr + i, cr[u]);
                     l2_fetch(g.cr + i + g.sz);        // plane c+1 <= mz-2
