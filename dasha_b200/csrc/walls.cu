@@ -64,12 +64,15 @@ public:
     double* tab = nullptr;
     cudaStream_t st = nullptr;
     long n = 0;
-    std::vector<double> hx;          // host staging of one padded 8-field array
     bool eq_set = false;
 
     ~WallEngine() override {
         if (pool) cudaFree(pool);
         if (tab) cudaFree(tab);
+        for (int b = 0; b < 2; ++b) {
+            if (pin[b] && small_buf.empty()) cudaFreeHost(pin[b]);
+            if (pev[b]) cudaEventDestroy(pev[b]);
+        }
     }
     walls::Core<GpuExec> core() { return walls::Core<GpuExec>{ex, d, t, par, a}; }
 
@@ -103,42 +106,100 @@ public:
             DASHA_CK(cudaMemcpy(a.rr0, r.data(), sizeof(double) * n, cudaMemcpyHostToDevice));
             DASHA_CK(cudaMemcpy(a.rr1, r.data(), sizeof(double) * n, cudaMemcpyHostToDevice));
         }
-        hx.assign(8 * (size_t)n, 0.);
         DASHA_CK(cudaStreamSynchronize(st));
         return Status::ok();
     }
 
-    // physical nodes of a host array in the reference's layout (leading dimensions ld1, ld2,
-    // (i+2) + ld1 (j + ld2 ((k+2) + (mz+4) m))) to / from the padded device array
-    void host_to_pad(const double* src, long ld1, long ld2, int nf, double* dst) const {
-        for (int m = 0; m < nf; ++m)
-            for (int k = 0; k < d.mz; ++k)
-                for (int j = 0; j < d.my; ++j)
-                    std::memcpy(dst + m * n + d.at(3, j + 1, k + 3), src + 2 + ld1 * (j + ld2 * ((k + 2) + (long)(d.mz + 4) * m)),
-                                sizeof(double) * d.mx);
+    // Physical nodes of a host array in the reference's layout (leading dimensions ld1, ld2, node
+    // (i+2) + ld1 (j + ld2 ((k+2) + (mz+4) m))) to / from a padded device array.  The rows move packed, in
+    // chunks through two pinned buffers (the host threads' gather or scatter of one chunk runs beside the DMA of the
+    // other) and a device array that is free meanwhile, which one kernel unpacks or packs: a copy of
+    // the padded arrays by one host thread and pageable memory took 17 ms each way at 129x72x101, this 5 and 6 ms.
+    // Eight fields of less than 4 MB go in one piece through pageable memory: to pin the buffers would take longer
+    // (20 ms more to set up a 41x25x33 context) than their transfers ever give back.
+    double* pin[2] = {nullptr, nullptr};
+    cudaEvent_t pev[2] = {nullptr, nullptr};
+    std::vector<double> small_buf;
+    static constexpr size_t PIN = size_t(8) << 20, SMALL = size_t(4) << 20;
+    long chunk_rows() const { return std::max(1L, (long)(PIN / sizeof(double)) / d.mx); }
+    Status pins() {
+        if (pev[1]) return Status::ok();
+        const size_t all = 8 * sizeof(double) * (size_t)d.mx * d.my * d.mz;
+        if (all < SMALL) {
+            small_buf.resize(all / sizeof(double));
+            pin[0] = pin[1] = small_buf.data();
+        }
+        for (int b = 0; b < 2; ++b) {
+            if (!pin[b]) DASHA_CK(cudaMallocHost(&pin[b], sizeof(double) * (size_t)chunk_rows() * d.mx));
+            if (!pev[b]) DASHA_CK(cudaEventCreateWithFlags(&pev[b], cudaEventDisableTiming));
+        }
+        return Status::ok();
     }
-    void pad_to_host(const double* src, long ld1, long ld2, int nf, double* dst) const {
-        for (int m = 0; m < nf; ++m)
-            for (int k = 0; k < d.mz; ++k)
-                for (int j = 0; j < d.my; ++j)
-                    std::memcpy(dst + 2 + ld1 * (j + ld2 * ((k + 2) + (long)(d.mz + 4) * m)), src + m * n + d.at(3, j + 1, k + 3),
-                                sizeof(double) * d.mx);
+    // host address of row r = j + my (k + mz m) of the caller's array
+    long row_at(long r, long ld1, long ld2) const {
+        const long j = r % d.my, q = r / d.my, k = q % d.mz, m = q / d.mz;
+        return 2 + ld1 * (j + ld2 * ((k + 2) + (long)(d.mz + 4) * m));
     }
-    Status upload(double* dev, int nf) {
-        DASHA_CK(cudaMemcpyAsync(dev, hx.data(), sizeof(double) * nf * n, cudaMemcpyHostToDevice, st));
+    Status upload(const double* src, long ld1, long ld2, int nf, double* dst, double* stage) {
+        Status s = pins();
+        if (s.code) return s;
+        const long rows = (long)nf * d.mz * d.my, step = chunk_rows();
+        int q = 0;
+        for (long r0 = 0; r0 < rows; r0 += step, ++q) {
+            const long r1 = std::min(rows, r0 + step);
+            double* h = pin[q & 1];
+            DASHA_CK(cudaEventSynchronize(pev[q & 1]));
+            HostPool::get().run(r1 - r0, [&](long a0, long a1) {
+                for (long r = a0; r < a1; ++r) std::memcpy(h + r * d.mx, src + row_at(r0 + r, ld1, ld2), sizeof(double) * d.mx);
+            });
+            DASHA_CK(cudaMemcpyAsync(stage + r0 * d.mx, h, sizeof(double) * (size_t)(r1 - r0) * d.mx, cudaMemcpyHostToDevice, st));
+            DASHA_CK(cudaEventRecord(pev[q & 1], st));
+        }
+        move(nf, [=] __device__(double* packed, double* padded) { *padded = *packed; }, stage, dst);
+        DASHA_CK(cudaGetLastError());
         DASHA_CK(cudaStreamSynchronize(st));
         return Status::ok();
     }
-    Status download(const double* dev, int nf) {
-        DASHA_CK(cudaMemcpyAsync(hx.data(), dev, sizeof(double) * nf * n, cudaMemcpyDeviceToHost, st));
-        DASHA_CK(cudaStreamSynchronize(st));
+    Status download(double* dst, long ld1, long ld2, int nf, double* src, double* stage) {
+        Status s = pins();
+        if (s.code) return s;
+        move(nf, [=] __device__(double* packed, double* padded) { *packed = *padded; }, stage, src);
+        DASHA_CK(cudaGetLastError());
+        const long rows = (long)nf * d.mz * d.my, step = chunk_rows();
+        auto copy = [&](long q) {
+            const long r0 = q * step, r1 = std::min(rows, r0 + step);
+            cudaError_t e = cudaMemcpyAsync(pin[q & 1], stage + r0 * d.mx, sizeof(double) * (size_t)(r1 - r0) * d.mx, cudaMemcpyDeviceToHost, st);
+            return e ? e : cudaEventRecord(pev[q & 1], st);
+        };
+        const long chunks = (rows + step - 1) / step;
+        DASHA_CK(copy(0));
+        for (long q = 0; q < chunks; ++q) {
+            if (q + 1 < chunks) DASHA_CK(copy(q + 1));
+            DASHA_CK(cudaEventSynchronize(pev[q & 1]));
+            const long r0 = q * step, r1 = std::min(rows, r0 + step);
+            const double* h = pin[q & 1];
+            HostPool::get().run(r1 - r0, [&](long a0, long a1) {
+                for (long r = a0; r < a1; ++r) std::memcpy(dst + row_at(r0 + r, ld1, ld2), h + r * d.mx, sizeof(double) * d.mx);
+            });
+        }
         return Status::ok();
+    }
+    // f(packed, padded) at every physical node of nf fields
+    template <class F>
+    void move(int nf, F f, double* packed, double* padded) {
+        const walls::Dims dd = d;
+        const long nn = n;
+        ex.run(core().physical(), [=] __device__(int jx, int jy, int jz) {
+            const long i = (jx - 3) + (long)dd.mx * ((jy - 1) + (long)dd.my * (jz - 3)), np = (long)dd.mx * dd.my * dd.mz;
+            const long c = dd.at(jx, jy, jz);
+            for (int m = 0; m < nf; ++m) f(packed + m * np + i, padded + m * nn + c);
+        });
     }
 
     // the equilibrium, then xresd as initia computes it (T:805-834): the state set to the
     // equilibrium, right(0, 1e-9, 1) with eta = 0 (foreta runs after it), xresd = the momentum rates
-    Status equilibrium_from_hx() {
-        Status s = upload(a.xm, 5);                   // rho0 bx0 by0 bz0 p0 staged in xm
+    Status equilibrium_from(const double* src, long ld1, long ld2) {
+        Status s = upload(src, ld1, ld2, 5, a.xm, a.xdif);   // rho0 bx0 by0 bz0 p0 by way of xm
         if (s.code) return s;
         double* eq[5] = {a.rhoi, a.bxi, a.byi, a.bzi, a.pri};
         for (int q = 0; q < 5; ++q) DASHA_CK(cudaMemcpyAsync(eq[q], a.xm + q * n, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
@@ -161,30 +222,23 @@ public:
     }
     Status set_equilibrium(const double* rho0, const double* b0, const double* p0, const double*) override {
         // z-profiles broadcast over x and y
-        std::fill(hx.begin(), hx.end(), 0.);
+        std::vector<double> e(5 * (size_t)n, 0.);
         const double* prof[5] = {rho0, b0, b0 + d.mz, b0 + 2 * d.mz, p0};
         for (int q = 0; q < 5; ++q)
             for (int k = 0; k < d.mz; ++k)
                 for (int j = 1; j <= d.my; ++j)
-                    for (int i = 3; i <= d.mx + 2; ++i) hx[q * n + d.at(i, j, k + 3)] = prof[q][k];
-        return equilibrium_from_hx();
+                    for (int i = 3; i <= d.mx + 2; ++i) e[q * n + d.at(i, j, k + 3)] = prof[q][k];
+        return equilibrium_from(e.data(), d.mxpr, d.my);
     }
     Status set_equilibrium_3d(const double* eq, long ld1, long ld2) override {
-        std::fill(hx.begin(), hx.end(), 0.);
-        host_to_pad(eq, ld1, ld2, 5, hx.data());
-        return equilibrium_from_hx();
+        return equilibrium_from(eq, ld1, ld2);
     }
     Status set_j0(const double*) override { return Status::err(DASHA_E_UNSUPPORTED, "J0 is a periodic-context option"); }
     Status set_state(const double* x, long ld1, long ld2) override {
-        std::fill(hx.begin(), hx.end(), 0.);
-        host_to_pad(x, ld1, ld2, 8, hx.data());
-        return upload(a.x, 8);
+        return upload(x, ld1, ld2, 8, a.x, a.xdif);
     }
     Status get_state(double* x, long ld1, long ld2) override {
-        Status s = download(a.x, 8);
-        if (s.code) return s;
-        pad_to_host(hx.data(), ld1, ld2, 8, x);
-        return Status::ok();
+        return download(x, ld1, ld2, 8, a.x, a.xdif);
     }
     Status setdt(double* dt, int* blowup) override {
         const double hundred = 100.;
@@ -208,10 +262,7 @@ public:
     Status current(double* cur, long ld1, long ld2) override {
         core().current();
         DASHA_CK(cudaGetLastError());
-        Status s = download(a.cur, 3);
-        if (s.code) return s;
-        pad_to_host(hx.data(), ld1, ld2, 3, cur);
-        return Status::ok();
+        return download(cur, ld1, ld2, 3, a.cur, a.xdif);
     }
     // right(t, 1e-9, 1) with xfold = x, as initia calls it; the state is restored afterwards
     // (the inflow driver writes the x-min rows of x)
@@ -220,10 +271,7 @@ public:
         core().right(tt, 1.e-9, 1);
         DASHA_CK(cudaMemcpyAsync(a.x, a.xfold, sizeof(double) * 8 * n, cudaMemcpyDeviceToDevice, st));
         DASHA_CK(cudaGetLastError());
-        Status s = download(a.xdif, 8);
-        if (s.code) return s;
-        pad_to_host(hx.data(), ld1, ld2, 8, xdif);
-        return Status::ok();
+        return download(xdif, ld1, ld2, 8, a.xdif, a.xm);
     }
     static Status no(const char* what) {
         return Status::err(DASHA_E_UNSUPPORTED, std::string(what) + " is not available on a bounded (periodic 0,0,0) context");
