@@ -1288,12 +1288,16 @@ public:
                      for (int m = 0; m < 8; ++m) cudaMemcpyAsync(dst[m], src[m], sizeof(T) * N, cudaMemcpyDeviceToDevice, st));
     }
     void zero8(T* const* f, int nf = 8) { for (int m = 0; m < nf; ++m) cudaMemsetAsync(f[m], 0, sizeof(T) * N, st); }
-    void axpby8(T* const* y, double b, T* const* x, double a) {
+    // tot and kap of the RK adjoint (k_adj_stage); null sig: tot = mu, null kap: none
+    void adj_stage(T* const* mu, T* const* sig, T* const* tot, T* const* kap, double a, double b) {
         if constexpr (std::is_same<T, double>::value) {
-            long nb = (N + 255) / 256;
-            F8<double> Y, Xv;
-            for (int m = 0; m < 8; ++m) { Y.f[m] = y[m]; Xv.f[m] = x[m]; }
-            DASHA_LAUNCH("a_axpby", 24.0 * N * 8, k_axpby8<<<nb, 256, 0, st>>>(N, Y, b, Xv, a));
+            F8<double> M{}, S2{}, Tt{}, Kp{};
+            for (int m = 0; m < 8; ++m) {
+                M.f[m] = mu[m]; Tt.f[m] = tot[m];
+                S2.f[m] = sig ? sig[m] : nullptr; Kp.f[m] = kap ? kap[m] : nullptr;
+            }
+            DASHA_LAUNCH("a_stage", 40.0 * N * 8,
+                         k_adj_stage<<<dim3((unsigned)((N + 255) / 256), 8), 256, 0, st>>>(N, M, S2, Tt, Kp, a, b));
         }
     }
 
@@ -1314,37 +1318,41 @@ public:
         }
     }
 
-    // transposed smoothing passes: n passes of nf (3 or 8) fields, kinds per field, in place
-    // on `a` using `b` as the other buffer; returns the buffer holding the result
-    T** adj_passes(T** a, T** b, int nf, int n, unsigned kinds3, bool fold_after) {
+    // grid of the column kernels of the adjoint over np planes, ZB planes a thread
+    dim3 adj_grid(int np, int zb, int nz = 1) const {
+        return dim3((unsigned)(((long)mx * my + 127) / 128), (unsigned)((np + zb - 1) / zb), (unsigned)nz);
+    }
+    // Planes a thread of the transposed passes, and of gather and curl: one.  Two and four share more of a
+    // thread's indices and column, but take 100-170 registers and leave too few loads in flight
+    // (128x64x128: 3-field pass 26, 30, 31 us with 1, 2, 4; gather 113, 172 us with 1, 2).
+    static constexpr int AZP = 1, AZG = 1;
+    // n transposed smoothing passes of nf (3 or 8) fields: in -> a -> b -> a ..., `in` unchanged unless it
+    // is a or b; returns the buffer holding the result
+    T** adj_passes(T* const* in, T** a, T** b, int nf, int n, bool eighth, bool fold_after) {
         if constexpr (std::is_same<T, double>::value) {
-            dim3 gf((mx + blk.x - 1) / blk.x, my, 1);
             for (int p = 0; p < n; ++p) {   // each transposed pass folds its input rows itself
+                const bool fold = fold_after && p == n - 1;
                 if (nf == 3) {
-                    FS<double, 3> in, out;
-                    for (int m = 0; m < 3; ++m) { in.f[m] = a[m]; out.f[m] = b[m]; }
-                    DASHA_LAUNCH("a_pass3", 6.0 * N * 8, k_adj_pass<3><<<grd, blk, 0, st>>>(g, adj_cr, in, out, kinds3));
+                    FS<double, 3> i3, o3;
+                    for (int m = 0; m < 3; ++m) { i3.f[m] = in[m]; o3.f[m] = a[m]; }
+                    if (eighth) DASHA_LAUNCH("a_pass3", 6.0 * N * 8, (k_adj_pass3<KIND_H, AZP><<<adj_grid(mz - 4, AZP), 128, 0, st>>>(g, i3, o3, fold)));
+                    else DASHA_LAUNCH("a_pass3", 7.0 * N * 8, (k_adj_pass3<0u, AZP><<<adj_grid(mz - 4, AZP), 128, 0, st>>>(g, i3, o3, fold)));
                 } else {
-                    FS<double, 4> in, out;
-                    for (int m = 0; m < 4; ++m) { in.f[m] = a[m]; out.f[m] = b[m]; }
-                    DASHA_LAUNCH("a_pass4", 8.0 * N * 8, k_adj_pass<4><<<grd, blk, 0, st>>>(g, adj_cr, in, out, 0u));
-                    for (int m = 0; m < 4; ++m) { in.f[m] = a[4 + m]; out.f[m] = b[4 + m]; }
-                    DASHA_LAUNCH("a_pass4", 8.0 * N * 8, k_adj_pass<4><<<grd, blk, 0, st>>>(g, adj_cr, in, out, KIND_B4));
+                    F8<double> i8, o8;
+                    for (int m = 0; m < 8; ++m) { i8.f[m] = in[m]; o8.f[m] = a[m]; }
+                    DASHA_LAUNCH("a_pass8", 17.0 * N * 8, (k_adj_pass8<KIND_B4, AZP><<<adj_grid(mz - 4, AZP, 2), 128, 0, st>>>(g, i8, o8, fold)));
                 }
+                in = a;
                 std::swap(a, b);
             }
-            if (fold_after) {
-                F8<double> fa{};
-                for (int m = 0; m < nf; ++m) fa.f[m] = a[m];
-                k_adj_fold_rows<<<dim3((mx + blk.x - 1) / blk.x, my, 1), blk, 0, st>>>(g, fa, nf);
-            }
+            return b;
         }
         return a;
     }
 
     // sigma = G'(S)^T kappa, G = avrg(right(.)); eta partials summed into *eta_acc (device)
     struct AdjScratch {
-        T *a8[8], *b8[8], *sb[8], *wq[8];
+        T *a8[8], *b8[8], *wq[4];
         T *e0[3], *e1[3], *et[3], *h0[3], *h1[3], *jb[3], *jt[3], *ub[3];
         double* etap;
         long netap;
@@ -1353,58 +1361,51 @@ public:
     void adj_rhs(T* const* Sx, T* const* kappa, T* const* sigma, AdjScratch& w) {
         if constexpr (std::is_same<T, double>::value) {
             launch_current(Sx);                       // curF = J of the stage state
-            for (int m = 0; m < 8; ++m) cudaMemcpyAsync(w.a8[m], kappa[m], sizeof(T) * N, cudaMemcpyDeviceToDevice, st);
-            T** rb = adj_passes(w.a8, w.b8, 8, 2, 0u, true);       // adjoint of the raw RHS (rows folded)
+            T** rb = adj_passes(kappa, w.a8, w.b8, 8, 2, false, true);   // adjoint of the raw RHS (rows folded)
             // induction: o_B = -curl(E_total)  ->  Et_bar = -curl^T(o_B)
             F3<double> ob3, et3;
             for (int m = 0; m < 3; ++m) { ob3.f[m] = rb[4 + m]; et3.f[m] = w.et[m]; }
-            DASHA_LAUNCH("a_curlT", 6.0 * N * 8, k_adj_curlT<<<grd, blk, 0, st>>>(g, ob3, et3, -1.0, 0));
+            DASHA_LAUNCH("a_curlT", 6.0 * N * 8, (k_adj_curlT<AZG><<<adj_grid(mz, AZG), 128, 0, st>>>(g, ob3, et3, -1.0, 0)));
             // E chain: 4 transposed avrgE passes -> adjoint of E0 (all nodes)
-            for (int m = 0; m < 3; ++m) cudaMemcpyAsync(w.e0[m], w.et[m], sizeof(T) * N, cudaMemcpyDeviceToDevice, st);
-            T** eb = adj_passes(w.e0, w.e1, 3, 4, 0u, false);
+            T** eb = adj_passes(w.et, w.e0, w.e1, 3, 4, false, false);
             T** hb = nullptr;
-            if (P.hall) {   // Hall chain: 5 transposed avrgh passes, then the rows of the Hall field (k_zeh) folded
-                for (int m = 0; m < 3; ++m) cudaMemcpyAsync(w.h0[m], w.et[m], sizeof(T) * N, cudaMemcpyDeviceToDevice, st);
-                hb = adj_passes(w.h0, w.h1, 3, 5, KIND_H, true);
-            }
-            zero8(w.sb);
+            if (P.hall)   // Hall chain: 5 transposed avrgh passes, then the rows of the Hall field (k_zeh) folded
+                hb = adj_passes(w.et, w.h0, w.h1, 3, 5, true, true);
             AdjPtw ap;
-            for (int m = 0; m < 8; ++m) { ap.s.f[m] = Sx[m]; ap.sb.f[m] = w.sb[m]; ap.wq.f[m] = w.wq[m]; }
+            for (int m = 0; m < 8; ++m) { ap.s.f[m] = Sx[m]; ap.sb.f[m] = sigma[m]; }
+            for (int m = 0; m < 4; ++m) ap.wq[m] = w.wq[m];
             for (int m = 0; m < 3; ++m) {
                 ap.j.f[m] = curF[m]; ap.eb.f[m] = eb[m]; ap.hb.f[m] = hb ? hb[m] : w.et[m];
-                ap.jb.f[m] = w.jb[m]; ap.ub.f[m] = w.ub[m];
+                ap.jb.f[m] = w.jb[m]; ap.ub.f[m] = w.ub[m]; ap.v.f[m] = w.jt[m];   // jt is free until the current chain
             }
             ap.ob[0] = rb[0]; ap.ob[1] = rb[1]; ap.ob[2] = rb[2]; ap.ob[3] = rb[3]; ap.ob[4] = rb[7];
             ap.etapart = w.etap;
             ap.hall = P.hall;
-            DASHA_LAUNCH("a_pointwise", 30.0 * N * 8, k_adj_pointwise<<<grd, blk, 0, st>>>(g, ap));
-            DASHA_LAUNCH("a_reduce", 0.0, k_reduce_add<<<1, 256, 0, st>>>(w.etap, w.netap, w.eta_acc));
+            DASHA_LAUNCH("a_velocity", 7.0 * N * 8, k_adj_velocity<<<(unsigned)((N + 255) / 256), 256, 0, st>>>(N, mz, g, ap.s, ap.v));
+            DASHA_LAUNCH("a_pointwise", 43.0 * N * 8, k_adj_pointwise<<<(unsigned)w.netap, 128, 0, st>>>(g, ap));
+            DASHA_LAUNCH("a_reduce", 0.0, k_reduce_add<<<1, 1024, 0, st>>>(w.etap, w.netap, w.eta_acc));
             AdjGat ag;
-            for (int m = 0; m < 8; ++m) { ag.s.f[m] = Sx[m]; ag.sb.f[m] = w.sb[m]; ag.wq.f[m] = w.wq[m]; }
+            for (int m = 0; m < 8; ++m) { ag.s.f[m] = Sx[m]; ag.sb.f[m] = sigma[m]; }
+            for (int m = 0; m < 4; ++m) ag.wq[m] = w.wq[m];
             for (int m = 0; m < 3; ++m) ag.ub.f[m] = w.ub[m];
             ag.ob[0] = rb[0]; ag.ob[1] = rb[1]; ag.ob[2] = rb[2]; ag.ob[3] = rb[3]; ag.ob[4] = rb[7];
-            DASHA_LAUNCH("a_gather", 25.0 * N * 8, k_adj_gather<<<grd, blk, 0, st>>>(g, ag));
+            DASHA_LAUNCH("a_gather", 25.0 * N * 8, (k_adj_gather<AZG><<<adj_grid(mz, AZG), 128, 0, st>>>(g, ag)));
             // current chain: 4 transposed avrgc passes, the curl's rows folded, curl^T into B
-            T** jt = adj_passes(w.jb, w.jt, 3, 4, 0u, true);
+            T** jt = adj_passes(w.jb, w.jt, w.e0, 3, 4, false, true);
             F3<double> jw, bo;
-            for (int m = 0; m < 3; ++m) { jw.f[m] = jt[m]; bo.f[m] = w.sb[4 + m]; }
-            DASHA_LAUNCH("a_curlT", 9.0 * N * 8, k_adj_curlT<<<grd, blk, 0, st>>>(g, jw, bo, 1.0, 1));
-            for (int m = 0; m < 8; ++m) cudaMemcpyAsync(sigma[m], w.sb[m], sizeof(T) * N, cudaMemcpyDeviceToDevice, st);
+            for (int m = 0; m < 3; ++m) { jw.f[m] = jt[m]; bo.f[m] = sigma[4 + m]; }
+            DASHA_LAUNCH("a_curlT", 9.0 * N * 8, (k_adj_curlT<AZG><<<adj_grid(mz, AZG), 128, 0, st>>>(g, jw, bo, 1.0, 1)));
         }
     }
 
-    long w_netap_max() const { return (long)grd.x * grd.y * grd.z; }
-    double* adj_cr = nullptr;   // radial coefficient field of the current adjoint call
+    long w_netap_max() const { return (N + 127) / 128; }
     bool adj_scratch(AdjBufs& B, AdjScratch& w) {
-        if constexpr (std::is_same<T, double>::value) {
-            if (!(adj_cr = B.take(N))) return false;
-            k_adj_cr<<<grd, blk, 0, st>>>(g, adj_cr);
-        }
         auto t8 = [&](T** a) { for (int m = 0; m < 8; ++m) if (!(a[m] = (T*)B.take(N))) return false; return true; };
         auto t3 = [&](T** a) { for (int m = 0; m < 3; ++m) if (!(a[m] = (T*)B.take(N))) return false; return true; };
-        if (!t8(w.a8) || !t8(w.b8) || !t8(w.sb) || !t8(w.wq)) return false;
+        if (!t8(w.a8) || !t8(w.b8)) return false;
+        for (auto& q : w.wq) if (!(q = (T*)B.take(N))) return false;
         if (!t3(w.e0) || !t3(w.e1) || !t3(w.et) || !t3(w.h0) || !t3(w.h1) || !t3(w.jb) || !t3(w.jt) || !t3(w.ub)) return false;
-        w.netap = (long)grd.x * grd.y * grd.z;
+        w.netap = w_netap_max();
         if (!(w.etap = B.take(w.netap)) || !(w.eta_acc = B.take(4))) return false;
         cudaMemsetAsync(w.eta_acc, 0, 4 * sizeof(double), st);
         return true;
@@ -1438,34 +1439,20 @@ public:
     // mu = F^T lambda (the post-step filter when step j filtered), then the RK4 stages in reverse:
     // kappa4 = dt/6 mu, sigma3 = G'(S3)^T kappa4, kappa3 = dt/3 mu + dt sigma3, ...,
     // lambda = mu + sigma0 + sigma1 + sigma2 + sigma3.
-    struct AdjVec { T *lam[8], *mu[8], *kap[8], *sig[8], *tot[8], *ta[8], *tb[8]; };
+    struct AdjVec { T *lam[8], *kap[8], *sig[8], *tot[8], *ta[8], *tb[8]; };
     void adj_step(T* const* Xn, T* const* s1, T* const* s2, T* const* s3, double dt, bool filtered, AdjVec& v,
                   AdjScratch& w) {
-        if (filtered) {
-            copy8(v.ta, v.lam);
-            T** r = adj_passes(v.ta, v.tb, 8, 2, 0u, false);
-            copy8(v.mu, r);
-        } else {
-            copy8(v.mu, v.lam);
-        }
-        copy8(v.tot, v.mu);                                    // lambda_X = mu + sum sigma
-        copy8(v.kap, v.mu);
-        axpby8(v.kap, dt / 6.0, v.mu, 0.0);                    // kappa4 = dt/6 mu
+        T* const* mu = filtered ? adj_passes(v.lam, v.ta, v.tb, 8, 2, false, false) : v.lam;
+        adj_stage(mu, nullptr, v.tot, v.kap, dt / 6.0, 0.0);   // lambda_X = mu + sum sigma; kappa4 = dt/6 mu
         adj_rhs(s3, v.kap, v.sig, w);                          // sigma3
-        axpby8(v.tot, 1.0, v.sig, 1.0);
-        axpby8(v.kap, 0.0, v.mu, dt / 3.0);                    // kappa3 = dt/3 mu + dt sigma3
-        axpby8(v.kap, 1.0, v.sig, dt);
+        adj_stage(mu, v.sig, v.tot, v.kap, dt / 3.0, dt);      // kappa3 = dt/3 mu + dt sigma3
         adj_rhs(s2, v.kap, v.sig, w);                          // sigma2
-        axpby8(v.tot, 1.0, v.sig, 1.0);
-        axpby8(v.kap, 0.0, v.mu, dt / 3.0);                    // kappa2 = dt/3 mu + dt/2 sigma2
-        axpby8(v.kap, 1.0, v.sig, dt / 2.0);
+        adj_stage(mu, v.sig, v.tot, v.kap, dt / 3.0, dt / 2.0);   // kappa2 = dt/3 mu + dt/2 sigma2
         adj_rhs(s1, v.kap, v.sig, w);                          // sigma1
-        axpby8(v.tot, 1.0, v.sig, 1.0);
-        axpby8(v.kap, 0.0, v.mu, dt / 6.0);                    // kappa1 = dt/6 mu + dt/2 sigma1
-        axpby8(v.kap, 1.0, v.sig, dt / 2.0);
+        adj_stage(mu, v.sig, v.tot, v.kap, dt / 6.0, dt / 2.0);   // kappa1 = dt/6 mu + dt/2 sigma1
         adj_rhs(Xn, v.kap, v.sig, w);                          // sigma0
-        axpby8(v.tot, 1.0, v.sig, 1.0);
-        copy8(v.lam, v.tot);
+        adj_stage(mu, v.sig, v.tot, nullptr, 0.0, 0.0);
+        std::swap_ranges(v.lam, v.lam + 8, v.tot);
     }
     // the seed lambda = dPhi/dX_N of the reconnected flux of the final state X_N
     void adj_seed(T* const* XN, T* const* lam) {
@@ -1509,7 +1496,7 @@ public:
             T *X0[8], *S1[8], *S2[8], *S3[8], *Xo[8], *Ac[8];
             AdjVec v;
             bool ok = take8(X0) && take8(S1) && take8(S2) && take8(S3) && take8(Xo) && take8(Ac) && take8(v.lam) &&
-                      take8(v.mu) && take8(v.kap) && take8(v.sig) && take8(v.tot) && take8(v.ta) && take8(v.tb);
+                      take8(v.kap) && take8(v.sig) && take8(v.tot) && take8(v.ta) && take8(v.tb);
             if (!ok) return Status::err(DASHA_E_NOMEM, "adjoint checkpoints do not fit in device memory");
             copy8(X0, X);
             if (keep_all) {
@@ -1561,7 +1548,8 @@ public:
             // gradients: eta, and psi through dBx = -Dz psi, dBz = Dx psi
             double* dpsi_d = B.take((size_t)mx * mz);
             if (!dpsi_d) return Status::err(DASHA_E_NOMEM, "adjoint scratch");
-            k_adj_psi<<<dim3((mx + blk.x - 1) / blk.x, mz, 1), blk, 0, st>>>(g, v.lam[4], v.lam[6], dpsi_d);
+            k_adj_ysum<<<dim3((mx + blk.x - 1) / blk.x, mz, 1), blk, 0, st>>>(g, v.lam[4], v.lam[6], w.jt[0], w.jt[1]);
+            k_adj_psi<<<dim3((mx + blk.x - 1) / blk.x, mz, 1), blk, 0, st>>>(g, w.jt[0], w.jt[1], dpsi_d);
             DASHA_CK(cudaGetLastError());
             std::vector<double> hp((size_t)mx * mz);
             DASHA_CK(cudaMemcpyAsync(hp.data(), dpsi_d, sizeof(double) * mx * mz, cudaMemcpyDeviceToHost, st));
