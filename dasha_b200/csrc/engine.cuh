@@ -772,12 +772,36 @@ public:
         DASHA_LAUNCH(tag, 6.0 * N * sizeof(T), (k_zcurl<T, ZVX, 8, 2, SIGN><<<gg, 256, ZC3c::smem(), st>>>(g, src, out, ch)));
     }
     // k_zhydro: one node per thread, tile 32 x 4, 1 plane in flight beyond c+2, 4 (FP32) or 3
-    // (FP64) CTAs per SM.  Measured (hydro ms per step, FP32 1024x512x1024 / FP64 512x256x512):
-    // float pairs, 8 rows, 1 CTA/SM 57.5 / -; pairs capped at 2 CTAs/SM (spills) 73.9 / -; one
-    // node per thread, 4 rows, 4 CTAs/SM 55.3 / -; 8 rows, 1 CTA/SM - / 16.6; 4 rows, 3 CTAs/SM
-    // 60.8 (pairs) / 12.8; 8 rows capped at 3 CTAs (spills) 66.5 / -
-    static constexpr int ZH_VX = 1, ZH_TY = 4, ZH_MINB = sizeof(T) == 4 ? 4 : 3;
-    using ZHc = ZH<T, ZH_VX, ZH_TY, 1>;
+    // (FP64) CTAs per SM; FP32 grids of some size take two nodes per thread, tile 64 x 6, 2 CTAs
+    // per SM (hydro_pairs).  Measured (us a launch, 512x256x256 / 256x128x256 FP32): one node, 4 rows, 4 CTAs
+    // 779 / 203; pairs, 4 rows, 3 CTAs 709 / 192; 4 rows, 2 CTAs 844 / 216; 5 rows, 2 CTAs 805 / 210;
+    // 6 rows, 2 CTAs 645 / 174; 7 rows, 2 CTAs (uneven over the schedulers) 722 / 204; 8 rows, 2 CTAs
+    // (128 registers, spills) 746 / 211; the register queue rotated by an unrolled march instead of moved 687 / 187.
+    // FP64 512x256x512, ms a step: 8 rows, 1 CTA 16.6; 4 rows, 3 CTAs 12.8.
+    static constexpr int ZH_TY = 4, ZH_MINB = sizeof(T) == 4 ? 4 : 3;
+    static constexpr int ZHP_TY = 6, ZHP_MINB = 2;
+    // Pairs halve the instructions per node (522 -> 332), but a plane's step is longer and its tile larger, so they
+    // lose where few tiles leave each CTA its latency (one node against pairs, us: 64x32x64 12.9 / 14.9, 6 tiles a
+    // plane; 100x44x77 21.0 / 21.1, 16; 128x64x96 27.7 / 27.1, 22; 128x128x64 35.4 / 33.3, 44) and where the tiles hang over
+    // the grid (32x200x50, half of each tile unused, 18.3 / 23.0; the gain at full tiles is about 1/7).  The rule is
+    // on the plane alone: every z-slab of a grid takes the grid's kernel.
+    bool hydro_pairs() const {
+        auto up = [](int n, int t) { return (long)((n + t - 1) / t) * t; };
+        const long one = up(mx, 32) * up(my, ZH_TY), two = up(mx, 64) * up(my, ZHP_TY);
+        return two >= 20L * 64 * ZHP_TY && 7 * two <= 8 * one;
+    }
+    template <int VX, int TY, int MINB>
+    cudaError_t hydro_attr() {
+        using Z = ZH<T, VX, TY, 1>;
+        cudaError_t e = cudaFuncSetAttribute(k_zhydro<T, VX, TY, 1, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)Z::smem());
+#ifndef DASHA_NO_TMA
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(k_zhydro_tma<T, VX, TY, 1, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)Z::smem_tma());
+#endif
+        return e;
+    }
     using ZEHc = ZEH<T, ZVX, 8, 2>;   // k_zeh: tile 32*ZVX x 8, 2 planes in flight beyond c+2
     using St3 = VStore<T, 3, ZVX>;
     using St4 = VStore<T, 4, ZVX>;
@@ -809,14 +833,9 @@ public:
         if ((e = cudaFuncSetAttribute(k_zeh<T, ZVX, 8, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)ZEHc::smem())))
             return e;
-        if ((e = cudaFuncSetAttribute(k_zhydro<T, ZH_VX, ZH_TY, 1, ZH_MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)ZHc::smem())))
-            return e;
-#ifndef DASHA_NO_TMA
-        if ((e = cudaFuncSetAttribute(k_zhydro_tma<T, ZH_VX, ZH_TY, 1, ZH_MINB>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ZHc::smem_tma())))
-            return e;
-#endif
+        if ((e = hydro_attr<1, ZH_TY, ZH_MINB>())) return e;
+        if constexpr (sizeof(T) == 4)
+            if ((e = hydro_attr<2, ZHP_TY, ZHP_MINB>())) return e;
         if ((e = cudaFuncSetAttribute(k_zcurl<T, ZVX, 8, 2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)ZC3c::smem())))
             return e;
@@ -962,13 +981,14 @@ public:
     const char* launch_err = nullptr;   // a launch that could not be set up (reported by stepon)
 #ifndef DASHA_NO_TMA
     // the five ring fields of k_zhydro as tensor maps, boxes of one ring plane (RS x NR x 1)
+    template <class Z>
     bool hydro_maps(const HydroIO<T>& io, ZhMaps& m) {
         EncodeTiledFn enc = encode_tiled();
         if (!enc) return false;
         const T* f[5] = {io.m1, io.m2, io.m3, io.dp, io.drho};
         const cuuint64_t dims[3] = {(cuuint64_t)mx, (cuuint64_t)my, (cuuint64_t)mz};
         const cuuint64_t strides[2] = {(cuuint64_t)g.sy * sizeof(T), (cuuint64_t)g.sz * sizeof(T)};
-        const cuuint32_t box[3] = {(cuuint32_t)ZHc::RS, (cuuint32_t)ZHc::NR, 1u};
+        const cuuint32_t box[3] = {(cuuint32_t)Z::RS, (cuuint32_t)Z::NR, 1u};
         const cuuint32_t estr[3] = {1u, 1u, 1u};
         const CUtensorMapDataType dt = sizeof(T) == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64;
         for (int q = 0; q < 5; ++q)
@@ -979,6 +999,26 @@ public:
         return true;
     }
 #endif
+    template <int VX, int TY, int MINB>
+    void launch_hydro(const HydroIO<T>& hio) {
+        using Z = ZH<T, VX, TY, 1>;
+        dim3 gh((mx + Z::TX - 1) / Z::TX, (my + TY - 1) / TY, 1);
+#ifndef DASHA_NO_TMA
+        const int chh = zchunk(gh.x * gh.y, (const void*)k_zhydro_tma<T, VX, TY, 1, MINB>, 32 * TY, Z::smem_tma());
+#else
+        const int chh = zchunk(gh.x * gh.y, (const void*)k_zhydro<T, VX, TY, 1, MINB>, 32 * TY, Z::smem());
+#endif
+        gh.z = (mz + chh - 1) / chh;
+#ifndef DASHA_NO_TMA
+        ZhMaps maps;
+        if (!hydro_maps<Z>(hio, maps)) launch_err = "cuTensorMapEncodeTiled failed for the hydro ring";
+        DASHA_LAUNCH("k_rhs_hydro", 16.0 * N * sizeof(T),
+                     (k_zhydro_tma<T, VX, TY, 1, MINB><<<gh, 32 * TY, Z::smem_tma(), st>>>(g, hio, chh, maps)));
+#else
+        DASHA_LAUNCH("k_rhs_hydro", 16.0 * N * sizeof(T),
+                     (k_zhydro<T, VX, TY, 1, MINB><<<gh, 32 * TY, Z::smem(), st>>>(g, hio, chh)));
+#endif
+    }
     void launch_current(T* const* xs) {
         T* bb[3] = {xs[4], xs[5], xs[6]};
         zcurl<1>("k_curl", src3(bb), f3(cur[0]));
@@ -1029,22 +1069,12 @@ public:
             hio.drho = xs[0]; hio.m1 = xs[1]; hio.m2 = xs[2]; hio.m3 = xs[3]; hio.dp = xs[7];
             hio.j1 = curF[0]; hio.j2 = curF[1]; hio.j3 = curF[2]; hio.b1 = xs[4]; hio.b2 = xs[5]; hio.b3 = xs[6];
             hio.out[0] = K[0]; hio.out[1] = K[1]; hio.out[2] = K[2]; hio.out[3] = K[3]; hio.out[4] = K[7];
-            dim3 gh((mx + ZHc::TX - 1) / ZHc::TX, (my + ZH_TY - 1) / ZH_TY, 1);
-#ifndef DASHA_NO_TMA
-            int chh = zchunk(gh.x * gh.y, (const void*)k_zhydro_tma<T, ZH_VX, ZH_TY, 1, ZH_MINB>, 32 * ZH_TY, ZHc::smem_tma());
-#else
-            int chh = zchunk(gh.x * gh.y, (const void*)k_zhydro<T, ZH_VX, ZH_TY, 1, ZH_MINB>, 32 * ZH_TY, ZHc::smem());
-#endif
-            gh.z = (mz + chh - 1) / chh;
-#ifndef DASHA_NO_TMA
-            ZhMaps maps;
-            if (!hydro_maps(hio, maps)) launch_err = "cuTensorMapEncodeTiled failed for the hydro ring";
-            DASHA_LAUNCH("k_rhs_hydro", 16.0 * N * sizeof(T),
-                         (k_zhydro_tma<T, ZH_VX, ZH_TY, 1, ZH_MINB><<<gh, 32 * ZH_TY, ZHc::smem_tma(), st>>>(g, hio, chh, maps)));
-#else
-            DASHA_LAUNCH("k_rhs_hydro", 16.0 * N * sizeof(T),
-                         (k_zhydro<T, ZH_VX, ZH_TY, 1, ZH_MINB><<<gh, 32 * ZH_TY, ZHc::smem(), st>>>(g, hio, chh)));
-#endif
+            if constexpr (sizeof(T) == 4) {
+                if (hydro_pairs()) launch_hydro<2, ZHP_TY, ZHP_MINB>(hio);
+                else launch_hydro<1, ZH_TY, ZH_MINB>(hio);
+            } else {
+                launch_hydro<1, ZH_TY, ZH_MINB>(hio);
+            }
         } else {
         dim3 gg(mx / ZTX, (my + 7) / 8, 1);
         int ch = zchunk(gg.x * gg.y, (const void*)k_zst2<T, 5, ZTX, 8, HMINB, OpHydro<T>>, ZTX * 8, ZS2<T, 5, ZTX, 8>::smem(true));

@@ -2,8 +2,11 @@
 // continuity, momentum (fluxes rho v_i v_j + (p - p0) delta_ij, J x B - xresd) and the pressure
 // equation, for the case without viscosity and diffusion; z-marching and register-blocked.
 //
-// A warp covers 32*VX consecutive x nodes (VX = 2 in FP32: float pairs), one row per warp, TY
-// warps per CTA.  Planes of m1, m2, m3, p - p0 and rho - rho0 (tile plus a 2-node x/y halo, no
+// A warp covers 32*VX consecutive x nodes, one row per warp, TY warps per CTA.  FP32 grids of some
+// size take VX = 2: issue slots bound the kernel (63 % used by one node per thread at 522 instructions a
+// node, where memory needs 333 of 779 us on 512x256x256), and a thread that owns two nodes loads float
+// pairs, forms and differences its fluxes as packed pairs with no register moves, and shares the tile's halo of
+// 1/rho among more nodes: 332 instructions a node, 779 -> 645 us.  Planes of m1, m2, m3, p - p0 and rho - rho0 (tile plus a 2-node x/y halo, no
 // corners) stream into an NS = D + 5 stage shared-memory ring with cp.async; the thread whose
 // copy landed turns rho - rho0 into 1/rho in place.  The five quantities of the own nodes for
 // planes c-2 .. c+2 stay in a register queue (the z stencil), so per plane a thread reads plane
@@ -40,7 +43,8 @@ struct ZH {
     static constexpr int OFF = EPC;                   // interior column offset (>= 2)
     static constexpr int RS = TX + 2 * OFF;
     static constexpr int NR = TY + 4;                 // rows y0-2 .. y0+TY+1
-    static constexpr int SP = NR * RS;
+    static constexpr int PL = NR * RS;                // nodes of one field-plane
+    static constexpr int SP = (PL * (int)sizeof(T) + 127) / 128 * 128 / (int)sizeof(T);   // its 128-byte aligned size
     static constexpr int NF = 5;                      // m1 m2 m3 dp ri
     static constexpr int NS = D + 5;
     static constexpr int CH = TX / EPC;
@@ -121,7 +125,7 @@ __device__ __forceinline__ void zhydro_body(const Geo<T>& g, const HydroIO<T>& i
                 T* stg = ring + (size_t)(p % NS) * NF * SP;
                 unsigned long long* bar = bars + p % NS;
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // after the stage's generic accesses
-                mbar_expect_tx(bar, (unsigned)(NF * SP * sizeof(T)));
+                mbar_expect_tx(bar, (unsigned)(NF * Z::PL * sizeof(T)));   // the boxes, not the padding
 #pragma unroll
                 for (int f = 0; f < NF; ++f) tma_load_3d(stg + f * SP, &maps->m[f], x0 - OFF, y0 - 2, p, bar);
             }
@@ -204,7 +208,15 @@ __device__ __forceinline__ void zhydro_body(const Geo<T>& g, const HydroIO<T>& i
                 if (!mbar_wait_bounded(bars + p % NS, (unsigned)(((p - (cA - 2)) / NS) & 1))) { late = true; break; }
                 const T r0 = T(g.rho0[p]);
                 T* ri = ring + (size_t)(p % NS) * NF * SP + 4 * SP;
-                for (int i = tid; i < SP; i += NT) ri[i] = recip(r0 + ri[i]);
+                if constexpr (VX == 2) {   // 16 bytes a thread: one pass of the CTA over the plane
+                    for (int i = EPC * tid; i < Z::PL; i += EPC * NT) {
+                        float4 q = *reinterpret_cast<float4*>(ri + i);
+                        q.x = recip(r0 + q.x); q.y = recip(r0 + q.y); q.z = recip(r0 + q.z); q.w = recip(r0 + q.w);
+                        *reinterpret_cast<float4*>(ri + i) = q;
+                    }
+                } else {
+                    for (int i = tid; i < Z::PL; i += NT) ri[i] = recip(r0 + ri[i]);
+                }
             }
             // these generic writes precede the boxes that refill the stage later
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -308,6 +320,65 @@ __device__ __forceinline__ void zhydro_body(const Geo<T>& g, const HydroIO<T>& i
                 const float2 r0 = d1p(P0, A2, B2, C2, D2), r1 = d1p(P1, A2, B2, C2, D2), r2 = d1p(P2, A2, B2, C2, D2);
                 o[0][0] -= r0.x; o[3][0] -= r0.y; o[1][0] -= r1.x; o[2][0] -= r1.y;
                 pz[0] = r2.x + T(g.dzp0[c]); dvv[0] -= r2.y;
+            }
+            } else if constexpr (std::is_same<T, float>::value && VX == 2) {
+            // FP32, two nodes per thread: the six quantities of a stencil node and their five-point
+            // differences as packed pairs over the two nodes (FADD2 / FMUL2 / FFMA2)
+            auto at2 = [&](int f, int off) { return *reinterpret_cast<const float2*>(pc + f * SP + me + off); };
+            auto own = [&](int s, int f) { return make_float2(zq[s][f][0], zq[s][f][1]); };
+            auto put = [](float (&t)[VX], float2 v) { t[0] = v.x; t[1] = v.y; };
+            // direction d of a node: m_d, F_d + dp (its own component), the other two F, dp, v_d
+            auto form = [](float2 md, float2 ma, float2 mb, float2 dp, float2 ri, float2 (&q)[6]) {
+                const float2 v = __fmul2_rn(md, ri);
+                q[0] = md; q[1] = __ffma2_rn(md, v, dp);
+                q[2] = __fmul2_rn(ma, v); q[3] = __fmul2_rn(mb, v);
+                q[4] = dp; q[5] = v;
+            };
+            // ---- x: the pairs at -2, 0, 2 hold the six nodes of the two stencils; a (fp - f0) and
+            // b (f0 - fm) share the difference of the two own nodes ----
+            {
+                float2 L[6], C[6], R[6], r[6];
+                form(at2(0, -2), at2(1, -2), at2(2, -2), at2(3, -2), at2(4, -2), L);
+                form(own(2, 0), own(2, 1), own(2, 2), own(2, 3), own(2, 4), C);
+                form(at2(0, 2), at2(1, 2), at2(2, 2), at2(3, 2), at2(4, 2), R);
+                const float2 A2 = make_float2(ax[0], ax[1]), B2 = make_float2(bx[0], bx[1]);
+                const float2 C2 = make_float2(cx[0], cx[1]), D2 = make_float2(dx[0], dx[1]);
+#pragma unroll
+                for (int u = 0; u < 6; ++u) {
+                    const float e = C[u].y - C[u].x;
+                    float2 t = __fmul2_rn(A2, make_float2(e, R[u].x - C[u].y));
+                    t = __ffma2_rn(B2, make_float2(C[u].x - L[u].y, e), t);
+                    t = __ffma2_rn(C2, __fadd2_rn(R[u], neg2(C[u])), t);
+                    r[u] = __ffma2_rn(D2, __fadd2_rn(C[u], neg2(L[u])), t);
+                }
+                put(o[0], neg2(r[0])); put(o[1], neg2(r[1])); put(o[2], neg2(r[2])); put(o[3], neg2(r[3]));
+                put(px, r[4]); put(dvv, neg2(r[5]));
+            }
+            auto sub = [&](float (&t)[VX], float2 v) { put(t, __fadd2_rn(make_float2(t[0], t[1]), neg2(v))); };
+            // ---- y ----
+            {
+                float2 Q[5][6], r[6];
+#pragma unroll
+                for (int s2 = 0; s2 < 5; ++s2) {
+                    const int off = (s2 - 2) * RS;
+                    if (s2 == 2) form(own(2, 1), own(2, 0), own(2, 2), own(2, 3), own(2, 4), Q[2]);
+                    else form(at2(1, off), at2(0, off), at2(2, off), at2(3, off), at2(4, off), Q[s2]);
+                }
+#pragma unroll
+                for (int u = 0; u < 6; ++u) r[u] = d1fc2(Q[0][u], Q[1][u], Q[2][u], Q[3][u], Q[4][u], bc2(ay), bc2(by), bc2(cy), bc2(dy));
+                sub(o[0], r[0]); sub(o[2], r[1]); sub(o[1], r[2]); sub(o[3], r[3]);
+                put(py, r[4]); sub(dvv, r[5]);
+            }
+            // ---- z, from the register queue ----
+            {
+                float2 Q[5][6], r[6];
+#pragma unroll
+                for (int s2 = 0; s2 < 5; ++s2) form(own(s2, 2), own(s2, 0), own(s2, 1), own(s2, 3), own(s2, 4), Q[s2]);
+#pragma unroll
+                for (int u = 0; u < 6; ++u) r[u] = d1fc2(Q[0][u], Q[1][u], Q[2][u], Q[3][u], Q[4][u], bc2(az), bc2(bz), bc2(cz), bc2(dz));
+                sub(o[0], r[0]); sub(o[3], r[1]); sub(o[1], r[2]); sub(o[2], r[3]);
+                put(pz, r[4]); pz[0] += T(g.dzp0[c]); pz[1] += T(g.dzp0[c]);
+                sub(dvv, r[5]);
             }
             } else {
             // ---- x ----
