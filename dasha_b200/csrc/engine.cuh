@@ -193,9 +193,11 @@ public:
     double* dtab = nullptr;      // 1-D tables in FP64
     double* red = nullptr;       // reduction scratch
     double* cfltab = nullptr;    // CFL rate tables: ich[mx+my+mz], vv[..], ih[..]
+    // bits of setdt's largest rate, two words taken in turn (a sweep clears the other one), then the
+    // blow-up flag: one copy reads all
+    unsigned long long* rate_bits = nullptr;
+    int rate_word = 0;
     int* flag = nullptr;         // blow-up flag
-    unsigned long long* rate_bits = nullptr;   // max CFL rate of the state, from the fused tap
-    bool rate_ok = false;        // rate_bits belongs to the current state (set by stepon)
     double* hpin = nullptr;      // pinned host scratch
     double* mpd = nullptr;       // the 11 mid-plane output fields (allocated on first use)
     Geo<T> g{};
@@ -237,7 +239,6 @@ public:
         if (dtab) cudaFree(dtab);
         if (red) cudaFree(red);
         if (cfltab) cudaFree(cfltab);
-        if (flag) cudaFree(flag);
         if (rate_bits) cudaFree(rate_bits);
         if (hpin) cudaFreeHost(hpin);
         if (mpd) cudaFree(mpd);
@@ -347,8 +348,9 @@ public:
         }
         nred = 2L * my * mz + my + 6L * mz + 64;
         DASHA_CK(cudaMalloc(&red, sizeof(double) * (nred + 16)));
-        DASHA_CK(cudaMalloc(&flag, sizeof(int)));
-        DASHA_CK(cudaMalloc(&rate_bits, sizeof(unsigned long long)));
+        DASHA_CK(cudaMalloc(&rate_bits, 24));
+        DASHA_CK(cudaMemsetAsync(rate_bits, 0, 24, st));
+        flag = (int*)(rate_bits + 2);
         DASHA_CK(cudaMemsetAsync(flag, 0, sizeof(int), st));
         DASHA_CK(cudaMallocHost(&hpin, sizeof(double) * 16));
 
@@ -371,7 +373,6 @@ public:
     }
 
     Status upload_eq() {
-        rate_ok = false;   // the CFL rate is of the totals: a new equilibrium invalidates it
         std::vector<double> h(16L * mz, 0.0);
         for (int k = 0; k < mz; ++k) {
             h[k] = rho0h[k]; h[mz + k] = b0h[0][k]; h[2 * mz + k] = b0h[1][k]; h[3 * mz + k] = b0h[2][k];
@@ -557,7 +558,6 @@ public:
     }
 
     Status state_in(const ChunkIn& fill) override {
-        rate_ok = false;
         Status s = stream_in(X, 8, true, fill);
         if (s.code) return s;
         if (KAHAN) for (int m = 0; m < 8; ++m) DASHA_CK(cudaMemsetAsync(C[m], 0, sizeof(T) * N, st));
@@ -604,7 +604,6 @@ public:
         }
         DASHA_CK(cudaMemsetAsync(flag, 0, sizeof(int), st));
         DASHA_CK(cudaStreamSynchronize(st));
-        rate_ok = false;
         return Status::ok();
     }
     Status set_state(const double* x, long ld1, long ld2) override { return state_in(gather(x, ld1, ld2)); }
@@ -817,7 +816,6 @@ public:
         if ((e = zp_attr1<4, KIND_B4, St4>())) return e;
         if ((e = zp_attr1<4, 0u, RK4>())) return e;
         if ((e = zp_attr1<4, KIND_B4, RK4>())) return e;
-        if ((e = zp_attr1<4, KIND_B4, WithCfl<St4, T, ZVX>>())) return e;
         if ((e = zp2_attr1<3, KIND_H, St3>())) return e;
         if constexpr (KAHAN) {
             if ((e = zp_attr1<4, 0u, VStore<T, 2, ZVX>, 1>())) return e;
@@ -825,7 +823,6 @@ public:
             if ((e = zp_attr1<4, KIND_P67, VStore<T, 2, ZVX>, 1>())) return e;
             if ((e = zp_attr1<4, 0u, VKF<T, 4, ZVX>, 2>())) return e;
             if ((e = zp_attr1<4, KIND_B4, VKF<T, 4, ZVX>, 2>())) return e;
-            if ((e = zp_attr1<4, KIND_B4, WithCfl<VKF<T, 4, ZVX>, T, ZVX>, 2>())) return e;
         }
         if ((e = cudaFuncSetAttribute(k_zst2<T, 5, ZTX, 8, HMINB, OpHydro<T>>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)ZS2<T, 5, ZTX, 8>::smem(true))))
@@ -867,32 +864,6 @@ public:
     // both xdif avrg passes of the raw RHS k, the second ending in the RK stage update: x =
     // stage state (or the step result at stage 4), base, acc, comp (FP32 Kahan compensation or
     // null)
-    // The fused CFL tap (CflTap, mhd_kernels.cuh) reading back the final state f, its maximum
-    // into rate_bits (cleared here, on the stream, before the tapped launch)
-    CflTap<T> cfl_tap(T* const* f) {
-        CflTap<T> c;
-        for (int m = 0; m < 8; ++m) c.x.f[m] = f[m];
-        const long nt = (long)mx + my + mz;
-        c.ich = cfltab; c.vv = cfltab + nt; c.ih = cfltab + 2 * nt;
-        c.rho0 = g.rho0; c.bx0 = g.bx0; c.by0 = g.by0; c.bz0 = g.bz0; c.p0 = g.p0;
-        c.gamma = P.gamma;
-        c.whistler = (P.dt_whistler && P.hall) ? P.di * 3.141592653589793 : 0.0;
-        c.mx = mx; c.my = my; c.mz = mz; c.sy = (unsigned)mx; c.sz = (unsigned)((long)mx * my);
-        c.out = rate_bits;
-        cudaMemsetAsync(rate_bits, 0, sizeof(unsigned long long), st);
-        return c;
-    }
-    template <class E>
-    WithCfl<E, T, ZVX> with_cfl(const E& e, T* const* f) {
-        WithCfl<E, T, ZVX> w;
-        static_cast<E&>(w) = e;
-        w.tap = cfl_tap(f);
-        w.best = 0.0;
-        return w;
-    }
-    // the tap reads 8 fields back per node: 4 finished by the launch before (DRAM), 4 just
-    // stored (L2)
-    double tap_bytes() const { return 4.0 * sizeof(T) * N; }
 
     // both xdif avrg passes of the raw RHS k, the second ending in the RK stage update: x =
     // stage state (or the step result at stage 4), base, acc, comp (FP32 Kahan compensation or
@@ -919,7 +890,7 @@ public:
 
     // avrgtt on the compensated FP32 state (X, C): pass 1 writes its increment of X - C into
     // t, pass 2 adds the two-pass increment to (X, C) in place with a Kahan step
-    void filter_compensated(T* const* t, bool tap = false) {
+    void filter_compensated(T* const* t) {
         for (int lo = 0; lo < 8; lo += 2) {   // pass 1 by field pairs: ring (x_a, x_b, comp_a, comp_b)
             SrcFields<T, 4> a;
             VStore<T, 2, ZVX> o;
@@ -935,8 +906,7 @@ public:
             VKF<T, 4, ZVX> e;
             for (int q = 0; q < 4; ++q) { d.f[q] = t[lo + q]; e.x[q] = X[lo + q]; e.comp[q] = C[lo + q]; }
             if (lo == 0) zp<4, 0u, 2>("k_zpv_F2", 20.0 * N * sizeof(T), d, e);
-            else if (!tap) zp<4, KIND_B4, 2>("k_zpv_F2", 20.0 * N * sizeof(T), d, e);
-            else zp<4, KIND_B4, 2>("k_zpv_F2", 20.0 * N * sizeof(T) + tap_bytes(), d, with_cfl(e, X));
+            else zp<4, KIND_B4, 2>("k_zpv_F2", 20.0 * N * sizeof(T), d, e);
         }
     }
 
@@ -1114,16 +1084,9 @@ public:
         (void)time;
         NvtxRange range("stepon");
         // stages 1..4: base = X, stage state in S, accumulator in A; both xdif smoothing
-        // passes run in one k_zpv2 launch per field pair that ends in the RK stage update.  When
-        // the post-step filter runs, its last launch (fields B, p) also takes the CFL rate of the
-        // new state for the next setdt (the tap leaves that launch's registers unchanged; on the
-        // RK stage-4 launch it would lower occupancy, so a step without the filter leaves setdt
-        // its own sweep).
+        // passes run in one k_zpv2 launch per field pair that ends in the RK stage update.
         const int every = P.filter_every > 0 ? P.filter_every : 1;
         const bool filt = nstep % every == 0;
-        // a z-slab takes setdt's rate by its own sweep (the tap would also read the ghost planes)
-        const bool tap = !cut();
-        rate_ok = false;
         hx(X, 8);
         for (int stage = 1; stage <= 4; ++stage) {
             launch_rhs_raw(stage == 1 ? X : S);
@@ -1136,15 +1099,14 @@ public:
             hx(X, 8);
             if constexpr (KAHAN) {
                 hx(C, 8);
-                filter_compensated(t, tap);
+                filter_compensated(t);
             } else {
                 pass8("k_zpv_F", 16.0, X, [&](int lo) { return st4(t, lo); });
                 hx(t, 8);
                 SrcFields<T, 4> a, b;
                 for (int q = 0; q < 4; ++q) { a.f[q] = t[q]; b.f[q] = t[4 + q]; }
                 zp<4, 0u>("k_zpv_F", 8.0 * N * sizeof(T), a, st4(S, 0));
-                if (tap) zp<4, KIND_B4>("k_zpv_F", 8.0 * N * sizeof(T) + tap_bytes(), b, with_cfl(st4(S, 4), S));
-                else zp<4, KIND_B4>("k_zpv_F", 8.0 * N * sizeof(T), b, st4(S, 4));
+                zp<4, KIND_B4>("k_zpv_F", 8.0 * N * sizeof(T), b, st4(S, 4));
                 for (int m = 0; m < 8; ++m) std::swap(X[m], S[m]);
             }
         }
@@ -1159,7 +1121,6 @@ public:
             launch_err = nullptr;
             return Status::err(DASHA_E_CUDA, e);
         }
-        rate_ok = filt && tap;
         return Status::ok();
     }
 
@@ -1183,12 +1144,11 @@ public:
             ka = own ? ga - z0 : -1;
             kb = own ? gb - z0 : -1;
         }
-        dim3 g2(1, my, mz);
+        const long nrows = (long)((my + DIAG_J - 1) / DIAG_J) * mz;
         DASHA_LAUNCH("k_diag_rows", 8.0 * N * sizeof(T),
-                     k_diag_rows<T><<<g2, 128, 0, st>>>(g, f8(X), wx, wy, wz, P.gamma, rows, klo, khi));
-        k_diag_flux<T><<<my, 128, 0, st>>>(g, f8(X), wx, fl, ka, kb);
-        k_diag_jext<T><<<mz, 128, 0, st>>>(g, f3(curF), my / 2, jext, klo, khi);
-        k_diag_final<<<1, 256, 0, st>>>(rows, (long)my * mz, fl, my, jext, mz, out, flag);
+                     k_diag_parts<T><<<(unsigned)(nrows + my + mz), 128, 0, st>>>(g, f8(X), f3(curF), wx, wy, wz, P.gamma, rows, fl,
+                                                                                  jext, klo, khi, ka, kb));
+        k_diag_final<<<1, 1024, 0, st>>>(rows, nrows, fl, my, jext, mz, out, flag);
         DASHA_CK(cudaGetLastError());
         return Status::ok();
     }
@@ -1213,31 +1173,24 @@ public:
 
     Status setdt(double* dt, int* blowup) override {
         NvtxRange range("setdt");
-        if (rate_ok) {   // the rate of this state was taken by the last stepon's final launch
-            DASHA_CK(cudaMemcpyAsync(hpin + 12, rate_bits, sizeof(double), cudaMemcpyDeviceToHost, st));
-            DASHA_CK(cudaMemcpyAsync(hpin + 13, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
-            DASHA_CK(cudaStreamSynchronize(st));
-            const double v = hpin[12];
-            int fl = 0;
-            std::memcpy(&fl, hpin + 13, sizeof(int));
-            *dt = (v != v) ? v : std::fmin(100.0, 1.0 / v);   // as k_reduce_rate
-            *blowup = fl;
-            return slab_reduce(dt, blowup);
-        }
-        dim3 g2(1, my, mz);
         const long nt = (long)mx + my + mz;
+        const int bx = (int)(((long)mx / (16 / (long)sizeof(T)) * (my - 1) + 255) / 256);
+        // enough CTAs for 8 on each SM, up to 8 planes to a thread (its x and y tables are read once)
+        const int planes = (int)std::max(1L, std::min(8L, (long)bx * mz / (8 * 148)));
+        const int nk = std::max(1, mz - 2 - g.kcfl0);
+        const int word = rate_word;
+        rate_word ^= 1;
         DASHA_LAUNCH("k_cfl", 8.0 * N * sizeof(T),
-                     k_cfl_rate<T><<<g2, 128, 0, st>>>(g, f8(X), cfltab, cfltab + nt, cfltab + 2 * nt, P.gamma,
-                                                       (P.dt_whistler && P.hall) ? P.di * 3.141592653589793 : 0.0, red));
-        k_reduce_rate<<<1, 256, 0, st>>>(red, (long)my * mz, red + nred + 12);
+                     k_cfl_rate<T><<<dim3(bx, (nk + planes - 1) / planes), 256, 0, st>>>(
+                         g, f8(X), cfltab, cfltab + nt, cfltab + 2 * nt, P.gamma,
+                         (P.dt_whistler && P.hall) ? P.di * 3.141592653589793 : 0.0, planes, rate_bits + word,
+                         rate_bits + (word ^ 1)));
         DASHA_CK(cudaGetLastError());
-        DASHA_CK(cudaMemcpyAsync(hpin + 12, red + nred + 12, sizeof(double), cudaMemcpyDeviceToHost, st));
-        int fl = 0;
-        DASHA_CK(cudaMemcpyAsync(hpin + 13, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
+        DASHA_CK(cudaMemcpyAsync(hpin + 12, rate_bits, 24, cudaMemcpyDeviceToHost, st));
         DASHA_CK(cudaStreamSynchronize(st));
-        std::memcpy(&fl, hpin + 13, sizeof(int));
-        *dt = hpin[12];
-        *blowup = fl;
+        const double v = hpin[12 + word];
+        *dt = (v != v) ? v : std::fmin(100.0, 1.0 / v);
+        std::memcpy(blowup, hpin + 14, sizeof(int));
         return slab_reduce(dt, blowup);
     }
     // a slab of a one-process-per-GPU run: the smallest dt and any blow-up of all slabs (the
@@ -1586,7 +1539,6 @@ public:
             double he = 0.0;
             DASHA_CK(cudaMemcpyAsync(&he, w.eta_acc, sizeof(double), cudaMemcpyDeviceToHost, st));
             copy8(X, X0);                                              // the context state is unchanged
-            rate_ok = false;
             DASHA_CK(cudaStreamSynchronize(st));
             *deta = he;
             std::memcpy(dpsi, hp.data(), sizeof(double) * mx * mz);

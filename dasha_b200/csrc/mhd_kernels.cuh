@@ -228,7 +228,7 @@ __device__ __forceinline__ double warp_sum(double v) {
 __device__ __forceinline__ double nanmax(double a, double b) { return (a != a || b != b) ? (a != a ? a : b) : fmax(a, b); }
 
 // The CFL rate of node c (totals = equilibrium profile at the node's plane + stored
-// perturbation), max over the three directions; shared by k_cfl_rate and the fused tap.
+// perturbation), max over the three directions.
 template <class T>
 __device__ __forceinline__ double cfl_node_rate(const F8<T>& x, long c, double r0, double bx0, double by0, double bz0,
                                                 double p0, double gamma, double whistler, double cx, double vx_,
@@ -246,273 +246,255 @@ __device__ __forceinline__ double cfl_node_rate(const F8<T>& x, long c, double r
     return nanmax(rx, nanmax(ry, rz));
 }
 
-// The fused form of setdt's sweep (survey row f3): the step's last launch, after it stores the
-// final B and p of a node (rho and rho v of the node were finished by the launch before it),
-// reads the node's 8 fields back and folds its CFL rate into a running maximum; at the end of
-// the launch each CTA adds its maximum with one atomicMax on the bits of a double (rates are
-// >= 0, so their bit patterns order as unsigned integers, and a NaN pattern lies above every
-// finite one: NaN wins as in k_cfl_rate).  The next dasha_setdt then needs no pass over the
-// state.  Region and formula as k_cfl_rate.
+// the 16 bytes of a field at p (aligned: rows are multiples of 4 values)
+__device__ __forceinline__ void load16(const float* p, float (&v)[4]) {
+    const float4 q = *reinterpret_cast<const float4*>(p);
+    v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+}
+__device__ __forceinline__ void load16(const double* p, double (&v)[2]) {
+    const double2 q = *reinterpret_cast<const double2*>(p);
+    v[0] = q.x; v[1] = q.y;
+}
+
+// setdt's sweep.  The rate needs FP64 (a division and two square roots a node: the FP64 pipe took 386 us for the
+// 33.5M nodes of 512x256x256 FP32, where memory needs 167), but only at nodes that can be the maximum: each
+// node first gets an upper bound in FP32, and cfl_node_rate runs where the bound reaches the largest rate known so far
+// (this warp's, and other CTAs' at the start), so the result is the full sweep's to the last bit.  The bound: rho, B and p
+// totals are formed in the field's precision; FP32 totals are off by 2^-24 (|background| + |total|), which is added to |B| and
+// |p| as 1e-6 |background| and kept below 8e-6 relative in rho by taking nodes with |rho| < |rho0| / 128
+// or outside 1e-10 .. 1e10 as unbounded; |B^2 + gamma p| <= B^2 + gamma |p|; the 1e-36 and 1e-25 cover
+// underflow; everything else is a sum of non-negative products whose roundings stay far below
+// the factor 1 + 3e-5.  NaN compares false and is evaluated, and NaN wins the maximum.
+// A thread owns 16 bytes of a row (4 FP32 or 2 FP64 nodes) and marches over `planes` planes, so
+// the x and y tables are read once; one atomicMax a CTA on the bits of the rate (rates are >= 0, a NaN pattern
+// lies above every finite one).  512x256x256 FP32 386 + 42 (a one-block reduction of the rows) -> 229 us,
+// 256x128x256 FP64 116 + 23 -> 108.  It also replaces a tap on the post-step filter's last launch, which
+// read the 8 fields back there and made that launch 500 us (512x256x256 FP32), 230 us (256x128x256 FP64) longer;
+// on 64x32x64 both ways take a step the same time.  Capped at 3 CTAs an SM (80 registers) 250 us, at 4 375.
 template <class T>
-struct CflTap {
-    F8<T> x;
-    const double *ich, *vv, *ih;   // per-axis tables, x | y | z concatenated
-    const double *rho0, *bx0, *by0, *bz0, *p0;
-    double gamma, whistler;
-    int mx, my, mz;
-    unsigned sy, sz;
-    unsigned long long* out;
-    __device__ __forceinline__ double rate(long i) const {
-        const unsigned n = (unsigned)i, k = n / sz, r = n - k * sz, j = r / sy, ix = r - j * sy;
-        if ((int)k > mz - 3 || (int)j > my - 2 || (int)ix > mx - 3) return 0.0;
-        const double *iy = ich + mx, *iz = ich + mx + my, *wy = vv + mx, *wz = vv + mx + my;
-        const double *hy = ih + mx, *hz = ih + mx + my;
-        return cfl_node_rate(x, i, rho0[k], bx0[k], by0[k], bz0[k], p0[k], gamma, whistler, ich[ix], vv[ix], ih[ix],
-                             iy[j], wy[j], hy[j], iz[k], wz[k], hz[k]);
-    }
-};
-
-// An epilogue with the tap: stores through Inner, then takes the rate of each stored node
-template <class Inner, class T, int VX>
-struct WithCfl : Inner {
-    CflTap<T> tap;
-    mutable double best;
-    using Pre = typename Inner::Pre;
-    __device__ __forceinline__ void take(long i) const {
+__global__ void __launch_bounds__(256) k_cfl_rate(Geo<T> g, F8<T> x, const double* ich, const double* vv, const double* ih,
+                                                  double gamma, double whistler, int planes, unsigned long long* out,
+                                                  unsigned long long* next) {
+    constexpr int V = 16 / (int)sizeof(T);
+    constexpr unsigned ALL = 0xffffffffu;
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *next = 0;   // the word the next sweep takes
+    const int nq = g.mx / V, id = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool on = id < nq * (g.my - 1);
+    const int jj = on ? id / nq : 0, i0 = on ? V * (id - jj * nq) : 0;
+    const double *ichy = ich + g.mx, *ichz = ichy + g.my, *vvy = vv + g.mx, *vvz = vvy + g.my, *ihy = ih + g.mx, *ihz = ihy + g.my;
+    float cx[V], ux[V], hx[V];
 #pragma unroll
-        for (int e = 0; e < VX; ++e) best = nanmax(best, tap.rate(i + e));
-    }
-    template <class V>
-    __device__ __forceinline__ void store(long i, const V& v, const Pre& p) const { Inner::store(i, v, p); take(i); }
-    template <class V>
-    __device__ __forceinline__ void wall(long i, const V& v) const { Inner::wall(i, v); take(i); }
-    template <class V>
-    __device__ __forceinline__ void store_rows(long i, bool wall, long ih, long iz, const V& v, const Pre& p) const {
-        Inner::store_rows(i, wall, ih, iz, v, p);
-        take(i);
-        if (wall) { take(ih); take(iz); }
-    }
-    // every thread of the CTA, after its last store
-    __device__ __forceinline__ void finish() const {
-        __shared__ double sh[32];
-        double v = best;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v = nanmax(v, __shfl_down_sync(0xffffffffu, v, o));
-        const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-        if (lane == 0) sh[wid] = v;
-        __syncthreads();
-        if (wid == 0) {
-            const int nw = (blockDim.x + 31) >> 5;
-            v = lane < nw ? sh[lane] : 0.0;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v = nanmax(v, __shfl_down_sync(0xffffffffu, v, o));
-            if (lane == 0 && v != 0.0) atomicMax(tap.out, (unsigned long long)__double_as_longlong(v));
-        }
-    }
-};
-
-template <class E, class = void>
-struct has_finish { static constexpr bool value = false; };
-template <class E>
-struct has_finish<E, decltype((void)&E::finish)> { static constexpr bool value = true; };
-
-template <class T>
-__global__ void k_cfl_rate(Geo<T> g, F8<T> x, const double* ich, const double* vv, const double* ih, double gamma,
-                           double whistler, double* partial) {
-    int jj = blockIdx.y, k = blockIdx.z;
+    for (int e = 0; e < V; ++e) { cx[e] = (float)ich[i0 + e]; ux[e] = fabsf((float)vv[i0 + e]); hx[e] = (float)ih[i0 + e]; }
+    const float cy = (float)ichy[jj], uy = fabsf((float)vvy[jj]), hy = (float)ihy[jj];
+    const float ga = fabsf((float)gamma), wh = fabsf((float)whistler);
+    const int ka = g.kcfl0 + blockIdx.y * planes, kb = min(ka + planes, g.mz - 2);
+    auto down = [](double b) { return b != b ? __int_as_float(0x7f800000) : __double2float_rd(b); };
     double best = 0.0;
-    const int nx = g.mx;
-    const double* ichx = ich;
-    const double* ichy = ich + nx;
-    const double* ichz = ich + nx + g.my;
-    const double* vvx = vv;
-    const double* vvy = vv + nx;
-    const double* vvz = vv + nx + g.my;
-    const double* ihx = ih;
-    const double* ihy = ih + nx;
-    const double* ihz = ih + nx + g.my;
-    if (k >= g.kcfl0 && k <= g.mz - 3 && jj <= g.my - 2) {
+    float thr = down(__longlong_as_double((long long)*(volatile unsigned long long*)out));
+    for (int k = ka; k < kb; ++k) {
         const double r0 = g.rho0[k], bx0 = g.bx0[k], by0 = g.by0[k], bz0 = g.bz0[k], p0 = g.p0[k];
-        const double cy = ichy[jj], vy_ = vvy[jj], cz = ichz[k], vz_ = vvz[k], hy = ihy[jj], hz = ihz[k];
-        for (int i = threadIdx.x; i <= g.mx - 3; i += blockDim.x) {
-            long c = (long)i + (long)jj * g.sy + (long)k * g.sz;
-            best = nanmax(best, cfl_node_rate(x, c, r0, bx0, by0, bz0, p0, gamma, whistler, ichx[i], vvx[i], ihx[i],
-                                              cy, vy_, hy, cz, vz_, hz));
+        const double czd = ichz[k], vzd = vvz[k], hzd = ihz[k];
+        const float cz = (float)czd, uz = fabsf((float)vzd), hz = (float)hzd;
+        const long c = (long)i0 + (long)jj * g.sy + (long)k * g.sz;
+        float est[V], top = -1.f;
+        {
+            T f[8][V];
+#pragma unroll
+            for (int m = 0; m < 8; ++m) load16(x.f[m] + c, f[m]);
+#pragma unroll
+            for (int e = 0; e < V; ++e) {
+                float r, b1, b2, b3, p;
+                bool ok = true;
+                if constexpr (sizeof(T) == 4) {
+                    const float R0 = (float)r0, X0 = (float)bx0, Y0 = (float)by0, Z0 = (float)bz0, P0 = (float)p0;
+                    r = fabsf(R0 + f[0][e]);
+                    ok = r >= 0.0078125f * fabsf(R0);
+                    b1 = fmaf(1e-6f, fabsf(X0), fabsf(X0 + f[4][e]));
+                    b2 = fmaf(1e-6f, fabsf(Y0), fabsf(Y0 + f[5][e]));
+                    b3 = fmaf(1e-6f, fabsf(Z0), fabsf(Z0 + f[6][e]));
+                    p = fmaf(1e-6f, fabsf(P0), fabsf(P0 + f[7][e]));
+                } else {
+                    r = fabsf((float)(r0 + f[0][e]));
+                    b1 = (float)(bx0 + f[4][e]); b2 = (float)(by0 + f[5][e]); b3 = (float)(bz0 + f[6][e]);
+                    p = fabsf((float)(p0 + f[7][e]));
+                }
+                const float ri = __fdividef(1.f, r);
+                const float bb = fmaf(b1, b1, fmaf(b2, b2, fmaf(b3, b3, 1e-36f)));
+                const float q = fmaf(ga, p, bb) * ri;
+                const float vf = q * rsqrtf(q);
+                const float w = wh != 0.f ? wh * (bb * rsqrtf(bb)) * ri : 0.f;
+                const float ex = fmaf(fmaf(fabsf((float)f[1][e]), ri, fmaf(w, hx[e], vf)), cx[e], ux[e]);
+                const float ey = fmaf(fmaf(fabsf((float)f[2][e]), ri, fmaf(w, hy, vf)), cy, uy);
+                const float ez = fmaf(fmaf(fabsf((float)f[3][e]), ri, fmaf(w, hz, vf)), cz, uz);
+                const float s = ex + ey + ez;   // NaN and infinity of any of the three
+                float b = fmaxf(ex, fmaxf(ey, ez)) * 1.00003f + 1e-25f;
+                if (!(ok && r >= 1e-10f && r <= 1e10f && s < 3e38f)) b = __int_as_float(0x7f800000);
+                est[e] = on && i0 + e <= g.mx - 3 ? b : -1.f;
+                top = fmaxf(top, est[e]);
+            }
         }
+        if (!__any_sync(ALL, top >= thr)) continue;
+        auto exact = [&](int e) {
+            const int i = i0 + e;
+            best = nanmax(best, cfl_node_rate(x, c + e, r0, bx0, by0, bz0, p0, gamma, whistler, ich[i], vv[i], ih[i],
+                                              ichy[jj], vvy[jj], ihy[jj], czd, vzd, hzd));
+        };
+        // the warp's highest bound first: its rate mostly rules the others out
+        const unsigned high = __reduce_max_sync(ALL, __float_as_uint(fmaxf(top, 0.f)));
+        if (top >= thr && __float_as_uint(top) == high) {
+            int m = 0;
+#pragma unroll
+            for (int e = V - 1; e >= 0; --e) if (est[e] == top) m = e;
+            exact(m);
+        }
+        thr = fmaxf(thr, __uint_as_float(__reduce_max_sync(ALL, __float_as_uint(down(best)))));
+#pragma unroll
+        for (int e = 0; e < V; ++e)
+            if (est[e] >= thr) exact(e);
+        thr = fmaxf(thr, __uint_as_float(__reduce_max_sync(ALL, __float_as_uint(down(best)))));
     }
-    __shared__ double sh[32];
+    __shared__ double sh[8];
     double v = best;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = nanmax(v, __shfl_down_sync(0xffffffffu, v, o));
-    int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0) sh[wid] = v;
+    for (int o = 16; o > 0; o >>= 1) v = nanmax(v, __shfl_down_sync(ALL, v, o));
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
     __syncthreads();
-    if (wid == 0) {
-        int nw = (blockDim.x + 31) >> 5;
-        v = lane < nw ? sh[lane] : 0.0;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v = nanmax(v, __shfl_down_sync(0xffffffffu, v, o));
-        if (lane == 0) partial[(long)blockIdx.z * gridDim.y + blockIdx.y] = v;
+    if (threadIdx.x == 0) {
+        for (int q = 1; q < 8; ++q) v = nanmax(v, sh[q]);
+        if (v != 0.0) atomicMax(out, (unsigned long long)__double_as_longlong(v));
     }
 }
 
-// dt = min(100, 1 / max rate) from the row partials, one block, fixed order
-static __global__ void k_reduce_rate(const double* partial, long n, double* out) {
-    double v = 0.0;
-    for (long q = threadIdx.x; q < n; q += blockDim.x) v = nanmax(v, partial[q]);
-    __shared__ double sh[32];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = nanmax(v, __shfl_down_sync(0xffffffffu, v, o));
-    int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+// sum over the CTA (at most 32 warps), in thread 0; sh is free again after the next barrier
+__device__ __forceinline__ double cta_sum(double v, double* sh) {
+    v = warp_sum(v);
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
     if (lane == 0) sh[wid] = v;
     __syncthreads();
-    if (wid == 0) {
-        int nw = (blockDim.x + 31) >> 5;
-        v = lane < nw ? sh[lane] : 0.0;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v = nanmax(v, __shfl_down_sync(0xffffffffu, v, o));
-        if (lane == 0) *out = (v != v) ? v : fmin(100.0, 1.0 / v);
-    }
+    v = threadIdx.x < nw ? sh[lane] : 0.;
+    return wid == 0 ? warp_sum(v) : v;
 }
 
-
-// Diagnostics partial sums per (j,k) row: mass, energy (trapezoid weights), and the
-// per-row extrema of J on the mid-y plane; partial layout [row][5]: mass, energy, jmax/jmin
-// handled separately.  Planes klo..khi count (a z-slab's own planes and the walls it holds);
-// the others give zero.
+// Diagnostics partial results, one launch for the three kinds of CTA (128 threads):
+//  - DIAG_J rows of a plane: mass and energy with the trapezoid weights, part[2 b], part[2 b + 1].  Planes klo..khi
+//    count (a z-slab's own planes and the walls it holds); the others give zero;
+//  - reconnected flux of a row j: sum_x sqrt(Bz(z=0)^2+eps^2)*wx, with Bz on the central plane ka (odd mz, kb = ka)
+//    or the mean of the two central planes ka, kb = ka + 1 (even mz); ka < 0: a z-slab that does not own
+//    the (first) central plane;
+//  - J extrema of a plane k's row my/2 (diagn t3dsdsc.f:1199-1214).
+// 16-byte loads, DIAG_J rows a CTA: an eighth of the partial results for the reduction that follows, and one launch
+// for three.  dasha_diagnostics of 256x128x256 FP32, its current included: 0.48 -> 0.38 ms.
+constexpr int DIAG_J = 8;
 template <class T>
-__global__ void k_diag_rows(Geo<T> g, F8<T> x, const double* wx, const double* wy, const double* wz,
-                            double gamma, double* part, int klo, int khi) {
-    int jj = blockIdx.y, k = blockIdx.z;
-    if (k < klo || k > khi) {
-        if (threadIdx.x == 0) {
-            long row = (long)k * gridDim.y + jj;
-            part[2 * row] = 0.;
-            part[2 * row + 1] = 0.;
-        }
-        return;
-    }
-    const double r0 = g.rho0[k], bx0 = g.bx0[k], by0 = g.by0[k], bz0 = g.bz0[k], p0 = g.p0[k];
-    double sm = 0., se = 0.;
-    for (int i = threadIdx.x; i < g.mx; i += blockDim.x) {
-        long c = (long)i + (long)jj * g.sy + (long)k * g.sz;
-        double rho = r0 + (double)x.f[0][c];
-        double m1 = x.f[1][c], m2 = x.f[2][c], m3 = x.f[3][c];
-        double b1 = bx0 + (double)x.f[4][c], b2 = by0 + (double)x.f[5][c], b3 = bz0 + (double)x.f[6][c];
-        double p = p0 + (double)x.f[7][c];
-        double vol = wx[i];
-        sm += rho * vol;
-        se += (0.5 * (m1 * m1 + m2 * m2 + m3 * m3) / rho + p / (gamma - 1.) + 0.5 * (b1 * b1 + b2 * b2 + b3 * b3)) * vol;
-    }
+__global__ void __launch_bounds__(128) k_diag_parts(Geo<T> g, F8<T> x, F3<T> cur, const double* wx, const double* wy,
+                                                    const double* wz, double gamma, double* part, double* fl, double* jext,
+                                                    int klo, int khi, int ka, int kb) {
+    constexpr int V = 16 / (int)sizeof(T);
     __shared__ double s1[32], s2[32];
-    sm = warp_sum(sm); se = warp_sum(se);
-    int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0) { s1[wid] = sm; s2[wid] = se; }
-    __syncthreads();
-    if (wid == 0) {
-        int nw = (blockDim.x + 31) >> 5;
-        sm = lane < nw ? s1[lane] : 0.;
-        se = lane < nw ? s2[lane] : 0.;
-        sm = warp_sum(sm); se = warp_sum(se);
-        if (lane == 0) {
-            long row = (long)k * gridDim.y + jj;
-            part[2 * row] = sm * wy[jj] * wz[k];
-            part[2 * row + 1] = se * wy[jj] * wz[k];
+    const int tid = threadIdx.x, nj = (g.my + DIAG_J - 1) / DIAG_J;
+    const long rows = (long)nj * g.mz;
+    const long b = blockIdx.x;
+    if (b < rows) {
+        const int k = (int)(b / nj), j0 = (int)(b - (long)k * nj) * DIAG_J, nr = min(DIAG_J, g.my - j0), nq = g.mx / V;
+        double sm = 0., se = 0.;
+        if (k >= klo && k <= khi) {
+            const double r0 = g.rho0[k], bx0 = g.bx0[k], by0 = g.by0[k], bz0 = g.bz0[k], p0 = g.p0[k];
+            for (int n = tid; n < nr * nq; n += blockDim.x) {
+                const int j = j0 + n / nq, i0 = V * (n % nq);
+                const long c = (long)i0 + (long)j * g.sy + (long)k * g.sz;
+                T f[8][V];
+#pragma unroll
+                for (int m = 0; m < 8; ++m) load16(x.f[m] + c, f[m]);
+                const double w = wy[j];
+#pragma unroll
+                for (int e = 0; e < V; ++e) {
+                    const double rho = r0 + (double)f[0][e], m1 = f[1][e], m2 = f[2][e], m3 = f[3][e];
+                    const double b1 = bx0 + (double)f[4][e], b2 = by0 + (double)f[5][e], b3 = bz0 + (double)f[6][e];
+                    const double p = p0 + (double)f[7][e], vol = wx[i0 + e] * w;
+                    sm += rho * vol;
+                    se += (0.5 * (m1 * m1 + m2 * m2 + m3 * m3) / rho + p / (gamma - 1.) + 0.5 * (b1 * b1 + b2 * b2 + b3 * b3)) * vol;
+                }
+            }
         }
-    }
-}
-
-// Reconnected flux partials per y row (one block per j): sum_x sqrt(Bz(z=0)^2+eps^2)*wx, with
-// Bz on the central plane ka (odd mz, kb = ka) or the mean of the two central planes ka, kb =
-// ka + 1 (even mz); ka < 0: a z-slab that does not own the (first) central plane.
-template <class T>
-__global__ void k_diag_flux(Geo<T> g, F8<T> x, const double* wx, double* part, int ka, int kb) {
-    int jj = blockIdx.x;
-    double s = 0.;
-    for (int i = threadIdx.x; i < g.mx && ka >= 0; i += blockDim.x) {
-        double bz;
-        if (ka == kb) {
-            bz = g.bz0[ka] + (double)x.f[6][(long)i + (long)jj * g.sy + (long)ka * g.sz];
-        } else {
-            double za = g.bz0[ka] + (double)x.f[6][(long)i + (long)jj * g.sy + (long)ka * g.sz];
-            double zb = g.bz0[kb] + (double)x.f[6][(long)i + (long)jj * g.sy + (long)kb * g.sz];
-            bz = 0.5 * (za + zb);
+        sm = cta_sum(sm, s1);
+        se = cta_sum(se, s2);
+        if (tid == 0) { part[2 * b] = sm * wz[k]; part[2 * b + 1] = se * wz[k]; }
+    } else if (b < rows + g.my) {
+        const int j = (int)(b - rows);
+        double s = 0.;
+        for (int i = tid; i < g.mx && ka >= 0; i += blockDim.x) {
+            const long c = (long)i + (long)j * g.sy;
+            double bz = g.bz0[ka] + (double)x.f[6][c + (long)ka * g.sz];
+            if (ka != kb) bz = 0.5 * (bz + (g.bz0[kb] + (double)x.f[6][c + (long)kb * g.sz]));
+            s += sqrt(bz * bz + 1e-20) * wx[i];
         }
-        s += sqrt(bz * bz + 1e-20) * wx[i];
-    }
-    __shared__ double sh[32];
-    s = warp_sum(s);
-    int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0) sh[wid] = s;
-    __syncthreads();
-    if (wid == 0) {
-        int nw = (blockDim.x + 31) >> 5;
-        s = lane < nw ? sh[lane] : 0.;
-        s = warp_sum(s);
-        if (lane == 0) part[jj] = s;
-    }
-}
-
-// J extrema on the mid-y plane (diagn t3dsdsc.f:1199-1214): one block per k row.
-template <class T>
-__global__ void k_diag_jext(Geo<T> g, F3<T> cur, int jm, double* part, int klo, int khi) {
-    int k = blockIdx.x;
-    double mx[3] = {-1e300, -1e300, -1e300}, mn[3] = {1e300, 1e300, 1e300};
-    for (int i = threadIdx.x; i < g.mx && k >= klo && k <= khi; i += blockDim.x) {
-        long c = (long)i + (long)jm * g.sy + (long)k * g.sz;
+        s = cta_sum(s, s1);
+        if (tid == 0) fl[j] = s;
+    } else {
+        const int k = (int)(b - rows - g.my), lane = tid & 31, wid = tid >> 5;
+        double mx[3] = {-1e300, -1e300, -1e300}, mn[3] = {1e300, 1e300, 1e300};
+        for (int i = tid; i < g.mx && k >= klo && k <= khi; i += blockDim.x) {
+            const long c = (long)i + (long)(g.my / 2) * g.sy + (long)k * g.sz;
+#pragma unroll
+            for (int m = 0; m < 3; ++m) {
+                const double v = cur.f[m][c];
+                mx[m] = fmax(mx[m], v);
+                mn[m] = fmin(mn[m], v);
+            }
+        }
+        __shared__ double sh[6][4];
 #pragma unroll
         for (int m = 0; m < 3; ++m) {
-            double v = cur.f[m][c];
-            mx[m] = fmax(mx[m], v);
-            mn[m] = fmin(mn[m], v);
+            const double a = warp_max(mx[m]), d = warp_min(mn[m]);
+            if (lane == 0) { sh[2 * m][wid] = a; sh[2 * m + 1][wid] = d; }
         }
-    }
-    __shared__ double sh[6][32];
-    int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-    for (int m = 0; m < 3; ++m) {
-        double a = warp_max(mx[m]), b = warp_min(mn[m]);
-        if (lane == 0) { sh[2 * m][wid] = a; sh[2 * m + 1][wid] = b; }
-    }
-    __syncthreads();
-    if (wid == 0) {
-        int nw = (blockDim.x + 31) >> 5;
-#pragma unroll
-        for (int m = 0; m < 3; ++m) {
-            double a = lane < nw ? sh[2 * m][lane] : -1e300;
-            double b = lane < nw ? sh[2 * m + 1][lane] : 1e300;
-            a = warp_max(a); b = warp_min(b);
-            if (lane == 0) { part[6 * k + 2 * m] = a; part[6 * k + 2 * m + 1] = b; }
+        __syncthreads();
+        if (tid < 6) {
+            double v = sh[tid][0];
+            for (int q = 1; q < 4; ++q) v = tid & 1 ? fmin(v, sh[tid][q]) : fmax(v, sh[tid][q]);
+            jext[6 * k + tid] = v;
         }
     }
 }
 
 // Final diagnostics reduction (one block, fixed order) -> out[9]; also raises the blow-up
-// flag when max Jy >= 1e7 (t3dsdsc.f:1232).
-static __global__ void k_diag_final(const double* rows, long nrows, const double* fl, int my, const double* jext, int mz,
-                             double* out, int* blowup) {
-    __shared__ double sh[2][32];
-    double sm = 0., se = 0.;
-    for (long q = threadIdx.x; q < nrows; q += blockDim.x) { sm += rows[2 * q]; se += rows[2 * q + 1]; }
-    sm = warp_sum(sm); se = warp_sum(se);
-    int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0) { sh[0][wid] = sm; sh[1][wid] = se; }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int nw = (blockDim.x + 31) >> 5;
-        double a = 0., b = 0.;
-        for (int w = 0; w < nw; ++w) { a += sh[0][w]; b += sh[1][w]; }
-        double f = 0.;
-        for (int j = 0; j < my; ++j) f += fl[j];
-        double e[6] = {-1e300, 1e300, -1e300, 1e300, -1e300, 1e300};
-        for (int k = 0; k < mz; ++k)
-            for (int m = 0; m < 3; ++m) {
-                e[2 * m] = fmax(e[2 * m], jext[6 * k + 2 * m]);
-                e[2 * m + 1] = fmin(e[2 * m + 1], jext[6 * k + 2 * m + 1]);
-            }
-        out[0] = a; out[1] = b; out[2] = f / my;
-        for (int q = 0; q < 6; ++q) out[3 + q] = e[q];
-        if (blowup && (fabs(e[2]) >= 1e7 || e[2] != e[2])) *blowup = 1;
+// flag when max Jy >= 1e7 (t3dsdsc.f:1232).  Every thread takes part in each sum and extremum: with the flux and the
+// extrema left to one thread and a row's result per (j, k) it took 105 us on 256x128x256, 138 us on 512x256x256.
+static __global__ void __launch_bounds__(1024) k_diag_final(const double* rows, long nrows, const double* fl, int my,
+                                                            const double* jext, int mz, double* out, int* blowup) {
+    __shared__ double sh[3][32], ex[6][32];
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    double sm = 0., se = 0., f = 0.;
+#pragma unroll 4
+    for (long q = tid; q < nrows; q += blockDim.x) {
+        const double2 v = *reinterpret_cast<const double2*>(rows + 2 * q);
+        sm += v.x;
+        se += v.y;
+    }
+    for (int j = tid; j < my; j += blockDim.x) f += fl[j];
+    double e[6] = {-1e300, 1e300, -1e300, 1e300, -1e300, 1e300};
+    for (int k = tid; k < mz; k += blockDim.x)
+#pragma unroll
+        for (int m = 0; m < 3; ++m) {
+            e[2 * m] = fmax(e[2 * m], jext[6 * k + 2 * m]);
+            e[2 * m + 1] = fmin(e[2 * m + 1], jext[6 * k + 2 * m + 1]);
+        }
+#pragma unroll
+    for (int q = 0; q < 6; ++q) {
+        const double v = q & 1 ? warp_min(e[q]) : warp_max(e[q]);
+        if (lane == 0) ex[q][wid] = v;
+    }
+    sm = cta_sum(sm, sh[0]);
+    se = cta_sum(se, sh[1]);
+    f = cta_sum(f, sh[2]);
+    if (wid == 0) {
+#pragma unroll
+        for (int q = 0; q < 6; ++q) e[q] = q & 1 ? warp_min(ex[q][lane]) : warp_max(ex[q][lane]);
+        if (tid == 0) {
+            out[0] = sm; out[1] = se; out[2] = f / my;
+            for (int q = 0; q < 6; ++q) out[3 + q] = e[q];
+            if (blowup && (fabs(e[2]) >= 1e7 || e[2] != e[2])) *blowup = 1;
+        }
     }
 }
 

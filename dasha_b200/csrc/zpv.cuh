@@ -590,7 +590,6 @@ __device__ __forceinline__ void zpv_body(const Geo<T>& g, const SrcFields<T, NF>
                 for (int e = 0; e < VX; ++e) { qm[u][f][e] = q0[u][f][e]; q0[u][f][e] = qp[u][f][e]; }
     }
     cp_async_wait<0>();
-    if constexpr (has_finish<Epi>::value) epi.finish();   // the fused CFL maximum (WithCfl)
 }
 
 template <class T, int NF, unsigned KINDS, int VX, int TYH, int RY, int D, class Epi, int MODE = 0>
