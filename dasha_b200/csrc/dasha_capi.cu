@@ -140,16 +140,20 @@ static int wait_status(dasha_ctx* c, int rc) {
     if (!hit) return rc;
     const unsigned int zero = 0;
     cudaMemcpyToSymbol(g_wait_timeout, &zero, sizeof(zero));
-    return fail(c, DASHA_E_CUDA, "a TMA ring wait ran out (k_zpv_tma / k_zhydro_tma)");
+    return fail(c, DASHA_E_CUDA, RING_WAIT_MSG);
 }
 #else
 static int wait_status(dasha_ctx*, int rc) { return rc; }
 #endif
 
+// `waits`: wait for the stream and look for ring waits that ran out.  dasha_stepon, which only enqueues, and dasha_setdt,
+// whose own copy brings the answer, do without on a whole-grid context: two waits with an idle GPU after each, 43 us
+// of a 661 us step on 64x32x64 FP64.
 template <class F>
-static int host_call(dasha_ctx* c, F body) {
+static int host_call(dasha_ctx* c, F body, bool waits = true) {
     try {
-        return wait_status(c, bounds_status(c, body()));
+        const int rc = bounds_status(c, body());
+        return waits ? wait_status(c, rc) : rc;
     } catch (const std::bad_alloc&) {
         return fail(c, DASHA_E_NOMEM, "host allocation failed");
     } catch (const std::exception& e) {
@@ -159,8 +163,8 @@ static int host_call(dasha_ctx* c, F body) {
     }
 }
 template <class F>
-static int engine_call(dasha_ctx* c, F call) {
-    return host_call(c, [&] { return from_status(c, call()); });
+static int engine_call(dasha_ctx* c, F call, bool waits = true) {
+    return host_call(c, [&] { return from_status(c, call()); }, waits);
 }
 
 extern "C" {
@@ -621,7 +625,7 @@ int dasha_setdt(dasha_ctx* c, double time, double* dt_out) {
     if (!c->state_set) return fail(c, DASHA_E_STATE, "no state set");
     int blowup = 0;
     double dt = 0.;
-    int rc = engine_call(c, [&] { return c->eng->setdt(&dt, &blowup); });
+    int rc = engine_call(c, [&] { return c->eng->setdt(&dt, &blowup); }, !c->eng->own_wait_status());
     if (rc) return rc;
     *dt_out = dt;
     return setdt_guards(c, dt, blowup);
@@ -632,7 +636,7 @@ int dasha_stepon(dasha_ctx* c, double time, double dt, int nstep) {
     if (int rc = slab_single_call(c)) return rc;
     if (!c->state_set) return fail(c, DASHA_E_STATE, "no state set");
     if (!(dt > 0.0) || !std::isfinite(dt)) return fail(c, DASHA_E_INVALID, "dt must be positive and finite");
-    return engine_call(c, [&] { return c->eng->stepon(time, dt, nstep); });
+    return engine_call(c, [&] { return c->eng->stepon(time, dt, nstep); }, !c->eng->own_wait_status());
 }
 
 int dasha_current(dasha_ctx* c, double* cur_f, long ld1, long ld2) {

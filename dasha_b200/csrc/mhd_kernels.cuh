@@ -274,10 +274,13 @@ __device__ __forceinline__ void load16(const double* p, double (&v)[2]) {
 template <class T>
 __global__ void __launch_bounds__(256) k_cfl_rate(Geo<T> g, F8<T> x, const double* ich, const double* vv, const double* ih,
                                                   double gamma, double whistler, int planes, unsigned long long* out,
-                                                  unsigned long long* next) {
+                                                  unsigned long long* next, const unsigned* waits, unsigned long long* late) {
     constexpr int V = 16 / (int)sizeof(T);
     constexpr unsigned ALL = 0xffffffffu;
-    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *next = 0;   // the word the next sweep takes
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
+        *next = 0;                        // the word the next sweep takes
+        *late = waits ? *waits : 0;       // ring waits that ran out in the launches before, for the same copy
+    }
     const int nq = g.mx / V, id = blockIdx.x * blockDim.x + threadIdx.x;
     const bool on = id < nq * (g.my - 1);
     const int jj = on ? id / nq : 0, i0 = on ? V * (id - jj * nq) : 0;
