@@ -127,12 +127,14 @@ __device__ __forceinline__ void adj_pass_body(const Geo<double>& g, const FS<dou
 template <unsigned KINDS, int ZB>
 static __global__ void __launch_bounds__(128, 8) k_adj_pass3(const __grid_constant__ Geo<double> g, const __grid_constant__ FS<double, 3> in,
                                                          const __grid_constant__ FS<double, 3> out, bool fold) {
+    wait_for_stream();
     adj_pass_body<3, KINDS, ZB>(g, in, out, fold);
 }
 // the 8 state-like fields: (rho, m) and (B, p) by blockIdx.z
 template <unsigned KINDS_B, int ZB>
 static __global__ void __launch_bounds__(128, 8) k_adj_pass8(const __grid_constant__ Geo<double> g, const __grid_constant__ F8<double> in,
                                                          const __grid_constant__ F8<double> out, bool fold) {
+    wait_for_stream();
     FS<double, 4> a, b;
     const int lo = 4 * (int)blockIdx.z;
 #pragma unroll
@@ -203,6 +205,7 @@ __device__ __forceinline__ void dt_column(const Geo<double>& g, const double* w,
 template <int ZB>
 static __global__ void __launch_bounds__(128) k_adj_curlT(const __grid_constant__ Geo<double> g, const __grid_constant__ F3<double> w,
                                                          const __grid_constant__ F3<double> out, double s, int accumulate) {
+    wait_for_stream();
     const DTCol t(g);
     if (!t.on) return;
     const int k0 = (int)blockIdx.y * ZB;
@@ -229,6 +232,7 @@ static __global__ void __launch_bounds__(128) k_adj_curlT(const __grid_constant_
 // v_d = m_d / rho at every node, for the divergence in k_adj_pointwise (13 divisions a node there otherwise)
 static __global__ void __launch_bounds__(256) k_adj_velocity(long n, int mz, const __grid_constant__ Geo<double> g,
                                                             const __grid_constant__ F8<double> s, const __grid_constant__ F3<double> v) {
+    wait_for_stream();
     const long c = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= n) return;
     const double ri = 1.0 / (g.rho0[c / g.sz] + s.f[0][c]);
@@ -258,6 +262,7 @@ struct AdjPtw {
 };
 
 static __global__ void __launch_bounds__(128, 4) k_adj_pointwise(const __grid_constant__ Geo<double> g, const __grid_constant__ AdjPtw a) {
+    wait_for_stream();
     const unsigned node = blockIdx.x * blockDim.x + threadIdx.x;
     const unsigned plane = (unsigned)g.sz, row = (unsigned)g.mx;
     double eta_acc = 0.0;
@@ -351,6 +356,7 @@ struct AdjGat {
 
 template <int ZB>
 static __global__ void __launch_bounds__(128, 4) k_adj_gather(const __grid_constant__ Geo<double> g, const __grid_constant__ AdjGat a) {
+    wait_for_stream();
     const DTCol t(g);
     if (!t.on) return;
     const int k0 = (int)blockIdx.y * ZB;
@@ -423,6 +429,7 @@ static __global__ void __launch_bounds__(128, 4) k_adj_gather(const __grid_const
 
 // *acc += sum(part[0..n)), one block, fixed order
 static __global__ void k_reduce_add(const double* part, long n, double* acc) {
+    wait_for_stream();
     double v = 0.0;
     for (long q = threadIdx.x; q < n; q += blockDim.x) v += part[q];
     __shared__ double sh[32];
@@ -442,6 +449,7 @@ static __global__ void k_reduce_add(const double* part, long n, double* acc) {
 static __global__ void __launch_bounds__(256) k_adj_stage(long n, const __grid_constant__ F8<double> mu, const __grid_constant__ F8<double> sig,
                                                          const __grid_constant__ F8<double> tot, const __grid_constant__ F8<double> kap,
                                                          double a, double b) {
+    wait_for_stream();
     const long c = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= n) return;
     const int m = blockIdx.y;

@@ -649,6 +649,11 @@ public:
         const int one = std::max(1, (int)(slots / gxy));
         return std::max(2, (mz + one - 1) / one);
     }
+    // launch.cuh on the context's stream; a z-slab's exchanges stay ordered by whole kernels
+    template <class... P, class... A>
+    void launch(void (*fn)(P...), dim3 grid, int threads, size_t smem, A&&... a) {
+        launch_overlapped(st, !halo, fn, grid, threads, smem, std::forward<A>(a)...);
+    }
     // radius-2 ring kernels (k_zst2): 32 x 8 columns per CTA
     static constexpr int ZTX = 32;
     // k_zpv tiling: a warp covers 32*ZVX x nodes (float pairs in FP32), a thread RY
@@ -720,11 +725,11 @@ public:
         if constexpr (zp_tma<NF>()) {
             ZpMaps maps;
             if (!zpv_maps<NF>(src, maps)) launch_err = "cuTensorMapEncodeTiled failed for a smoothing pass";
-            DASHA_LAUNCH(tag, bytes, (zpv_tma_fn<NF, KINDS, Epi, MODE>()<<<gg, 32 * ZC<NF>::TYH, Z::smem_tma(), st>>>(g, src, epi, ch, maps)));
+            DASHA_LAUNCH(tag, bytes, launch(zpv_tma_fn<NF, KINDS, Epi, MODE>(), gg, 32 * ZC<NF>::TYH, Z::smem_tma(), g, src, epi, ch, maps));
         } else
 #endif
         {
-            DASHA_LAUNCH(tag, bytes, (zpv_fn<NF, KINDS, Epi, MODE>()<<<gg, 32 * ZC<NF>::TYH, Z::smem(), st>>>(g, src, epi, ch)));
+            DASHA_LAUNCH(tag, bytes, launch(zpv_fn<NF, KINDS, Epi, MODE>(), gg, 32 * ZC<NF>::TYH, Z::smem(), g, src, epi, ch));
         }
     }
     template <int NF, unsigned KINDS, class Epi, int MODE = 0>
@@ -764,7 +769,7 @@ public:
         dim3 gg((mx + Z::TX - 1) / Z::TX, (my + ZC2<NF>::TY - 1) / ZC2<NF>::TY, 1);
         int ch = zchunk(gg.x * gg.y, (const void*)zpv2_fn<NF, KINDS, Epi>(), 32 * Z::NW, Z::smem());
         gg.z = (mz + ch - 1) / ch;
-        DASHA_LAUNCH(tag, bytes, (zpv2_fn<NF, KINDS, Epi>()<<<gg, 32 * Z::NW, Z::smem(), st>>>(g, src, epi, ch)));
+        DASHA_LAUNCH(tag, bytes, launch(zpv2_fn<NF, KINDS, Epi>(), gg, 32 * Z::NW, Z::smem(), g, src, epi, ch));
     }
     template <int NF, unsigned KINDS, class Epi>
     static cudaError_t zp2_attr1() {
@@ -778,7 +783,7 @@ public:
         dim3 gg((mx + ZC3c::TX - 1) / ZC3c::TX, (my + 7) / 8, 1);
         int ch = zchunk(gg.x * gg.y, (const void*)k_zcurl<T, ZVX, 8, 2, SIGN>, 256, ZC3c::smem());
         gg.z = (mz + ch - 1) / ch;
-        DASHA_LAUNCH(tag, 6.0 * N * sizeof(T), (k_zcurl<T, ZVX, 8, 2, SIGN><<<gg, 256, ZC3c::smem(), st>>>(g, src, out, ch)));
+        DASHA_LAUNCH(tag, 6.0 * N * sizeof(T), launch(k_zcurl<T, ZVX, 8, 2, SIGN>, gg, 256, ZC3c::smem(), g, src, out, ch));
     }
     // k_zhydro: one node per thread, tile 32 x 4, 1 plane in flight beyond c+2, 4 (FP32) or 3
     // (FP64) CTAs per SM; FP32 grids of some size take two nodes per thread, tile 64 x 6, 2 CTAs
@@ -993,10 +998,10 @@ public:
         ZhMaps maps;
         if (!hydro_maps<Z>(hio, maps)) launch_err = "cuTensorMapEncodeTiled failed for the hydro ring";
         DASHA_LAUNCH("k_rhs_hydro", 16.0 * N * sizeof(T),
-                     (k_zhydro_tma<T, VX, TY, 1, MINB><<<gh, 32 * TY, Z::smem_tma(), st>>>(g, hio, chh, maps)));
+                     launch(k_zhydro_tma<T, VX, TY, 1, MINB>, gh, 32 * TY, Z::smem_tma(), g, hio, chh, maps));
 #else
         DASHA_LAUNCH("k_rhs_hydro", 16.0 * N * sizeof(T),
-                     (k_zhydro<T, VX, TY, 1, MINB><<<gh, 32 * TY, Z::smem(), st>>>(g, hio, chh)));
+                     launch(k_zhydro<T, VX, TY, 1, MINB>, gh, 32 * TY, Z::smem(), g, hio, chh));
 #endif
     }
     void launch_current(T* const* xs) {
@@ -1004,7 +1009,7 @@ public:
         zcurl<1>("k_curl", src3(bb), f3(cur[0]));
         hx(cur[0], 3);
         curF = passes3<0u>("k_zpv_J", cur[0], cur[1], 4, false);
-        if (P.j0_mode == 1) DASHA_LAUNCH("k_add_j0", 6.0 * N * sizeof(T), k_add_j0<T><<<grd, blk, 0, st>>>(g, f3(curF)));
+        if (P.j0_mode == 1) DASHA_LAUNCH("k_add_j0", 6.0 * N * sizeof(T), launch(k_add_j0<T>, grd, (int)blk.x, 0, g, f3(curF)));
     }
 
     // E_total and the raw RHS of state xs into K (wall rows applied)
@@ -1022,10 +1027,10 @@ public:
             dim3 ge((mx + ZEHc::TX - 1) / ZEHc::TX, (my + 7) / 8, 1);
             int che = zchunk(ge.x * ge.y, (const void*)k_zeh<T, ZVX, 8, 2>, 256, ZEHc::smem());
             ge.z = (mz + che - 1) / che;
-            DASHA_LAUNCH("k_efield_hall", 17.0 * N * sizeof(T), (k_zeh<T, ZVX, 8, 2><<<ge, 256, ZEHc::smem(), st>>>(g, eh, che)));
+            DASHA_LAUNCH("k_efield_hall", 17.0 * N * sizeof(T), launch(k_zeh<T, ZVX, 8, 2>, ge, 256, ZEHc::smem(), g, eh, che));
             hx(Hh[0], 3);
         } else {
-            DASHA_LAUNCH("k_efield", 13.0 * N * sizeof(T), k_efield<T><<<grd, blk, 0, st>>>(g, f8(xs), f3(curF), f3(E[0])));
+            DASHA_LAUNCH("k_efield", 13.0 * N * sizeof(T), launch(k_efield<T>, grd, (int)blk.x, 0, g, f8(xs), f3(curF), f3(E[0])));
         }
         hx(E[0], 3);
         if (P.hall) {
@@ -1065,7 +1070,7 @@ public:
         oh.out[0] = K[0]; oh.out[1] = K[1]; oh.out[2] = K[2]; oh.out[3] = K[3]; oh.out[4] = K[7];
         oh.j1 = curF[0]; oh.j2 = curF[1]; oh.j3 = curF[2]; oh.b1 = xs[4]; oh.b2 = xs[5]; oh.b3 = xs[6];
         DASHA_LAUNCH("k_rhs_hydro", 16.0 * N * sizeof(T),
-                     (k_zst2<T, 5, ZTX, 8, HMINB, OpHydro<T>><<<gg, ZTX * 8, ZS2<T, 5, ZTX, 8>::smem(true), st>>>(g, sh, oh, ch)));
+                     launch(k_zst2<T, 5, ZTX, 8, HMINB, OpHydro<T>>, gg, ZTX * 8, ZS2<T, 5, ZTX, 8>::smem(true), g, sh, oh, ch));
         }
         T* kb[3] = {K[4], K[5], K[6]};
         zcurl<-1>("k_rhs_induction", src3(Ef), f3(kb));
@@ -1156,9 +1161,9 @@ public:
         }
         const long nrows = (long)((my + DIAG_J - 1) / DIAG_J) * mz;
         DASHA_LAUNCH("k_diag_rows", 8.0 * N * sizeof(T),
-                     k_diag_parts<T><<<(unsigned)(nrows + my + mz), 128, 0, st>>>(g, f8(X), f3(curF), wx, wy, wz, P.gamma, rows, fl,
+                     launch(k_diag_parts<T>, (unsigned)(nrows + my + mz), 128, 0, g, f8(X), f3(curF), wx, wy, wz, P.gamma, rows, fl,
                                                                                   jext, klo, khi, ka, kb));
-        k_diag_final<<<1, 1024, 0, st>>>(rows, nrows, fl, my, jext, mz, out, flag);
+        launch(k_diag_final, 1, 1024, 0, rows, nrows, fl, my, jext, mz, out, flag);
         DASHA_CK(cudaGetLastError());
         return Status::ok();
     }
@@ -1191,8 +1196,7 @@ public:
         const int word = rate_word;
         rate_word ^= 1;
         DASHA_LAUNCH("k_cfl", 8.0 * N * sizeof(T),
-                     k_cfl_rate<T><<<dim3(bx, (nk + planes - 1) / planes), 256, 0, st>>>(
-                         g, f8(X), cfltab, cfltab + nt, cfltab + 2 * nt, P.gamma,
+                     launch(k_cfl_rate<T>, dim3(bx, (nk + planes - 1) / planes), 256, 0, g, f8(X), cfltab, cfltab + nt, cfltab + 2 * nt, P.gamma,
                          (P.dt_whistler && P.hall) ? P.di * 3.141592653589793 : 0.0, planes, rate_bits + word,
                          rate_bits + (word ^ 1), waits, rate_bits + 3));
         DASHA_CK(cudaGetLastError());
@@ -1237,7 +1241,7 @@ public:
         launch_current(X);
         F8<T> cz;
         for (int m = 0; m < 8; ++m) cz.f[m] = KAHAN ? C[m] : nullptr;
-        k_midplane<T><<<dim3((mx + 127) / 128, mz), 128, 0, st>>>(g, my / 2, f8(X), cz, f3(curF), mpd);
+        launch(k_midplane<T>, dim3((mx + 127) / 128, mz), 128, 0, g, my / 2, f8(X), cz, f3(curF), mpd);
         DASHA_CK(cudaGetLastError());
         DASHA_CK(cudaMemcpyAsync(outh, mpd, sizeof(double) * 11 * (size_t)mx * mz, cudaMemcpyDeviceToHost, st));
         DASHA_CK(cudaStreamSynchronize(st));
@@ -1296,7 +1300,7 @@ public:
                 S2.f[m] = sig ? sig[m] : nullptr; Kp.f[m] = kap ? kap[m] : nullptr;
             }
             DASHA_LAUNCH("a_stage", 40.0 * N * 8,
-                         k_adj_stage<<<dim3((unsigned)((N + 255) / 256), 8), 256, 0, st>>>(N, M, S2, Tt, Kp, a, b));
+                         launch(k_adj_stage, dim3((unsigned)((N + 255) / 256), 8), 256, 0, N, M, S2, Tt, Kp, a, b));
         }
     }
 
@@ -1334,12 +1338,12 @@ public:
                 if (nf == 3) {
                     FS<double, 3> i3, o3;
                     for (int m = 0; m < 3; ++m) { i3.f[m] = in[m]; o3.f[m] = a[m]; }
-                    if (eighth) DASHA_LAUNCH("a_pass3", 6.0 * N * 8, (k_adj_pass3<KIND_H, AZP><<<adj_grid(mz - 4, AZP), 128, 0, st>>>(g, i3, o3, fold)));
-                    else DASHA_LAUNCH("a_pass3", 7.0 * N * 8, (k_adj_pass3<0u, AZP><<<adj_grid(mz - 4, AZP), 128, 0, st>>>(g, i3, o3, fold)));
+                    if (eighth) DASHA_LAUNCH("a_pass3", 6.0 * N * 8, (launch(k_adj_pass3<KIND_H, AZP>, adj_grid(mz - 4, AZP), 128, 0, g, i3, o3, fold)));
+                    else DASHA_LAUNCH("a_pass3", 7.0 * N * 8, (launch(k_adj_pass3<0u, AZP>, adj_grid(mz - 4, AZP), 128, 0, g, i3, o3, fold)));
                 } else {
                     F8<double> i8, o8;
                     for (int m = 0; m < 8; ++m) { i8.f[m] = in[m]; o8.f[m] = a[m]; }
-                    DASHA_LAUNCH("a_pass8", 17.0 * N * 8, (k_adj_pass8<KIND_B4, AZP><<<adj_grid(mz - 4, AZP, 2), 128, 0, st>>>(g, i8, o8, fold)));
+                    DASHA_LAUNCH("a_pass8", 17.0 * N * 8, (launch(k_adj_pass8<KIND_B4, AZP>, adj_grid(mz - 4, AZP, 2), 128, 0, g, i8, o8, fold)));
                 }
                 in = a;
                 std::swap(a, b);
@@ -1364,7 +1368,7 @@ public:
             // induction: o_B = -curl(E_total)  ->  Et_bar = -curl^T(o_B)
             F3<double> ob3, et3;
             for (int m = 0; m < 3; ++m) { ob3.f[m] = rb[4 + m]; et3.f[m] = w.et[m]; }
-            DASHA_LAUNCH("a_curlT", 6.0 * N * 8, (k_adj_curlT<AZG><<<adj_grid(mz, AZG), 128, 0, st>>>(g, ob3, et3, -1.0, 0)));
+            DASHA_LAUNCH("a_curlT", 6.0 * N * 8, (launch(k_adj_curlT<AZG>, adj_grid(mz, AZG), 128, 0, g, ob3, et3, -1.0, 0)));
             // E chain: 4 transposed avrgE passes -> adjoint of E0 (all nodes)
             T** eb = adj_passes(w.et, w.e0, w.e1, 3, 4, false, false);
             T** hb = nullptr;
@@ -1380,20 +1384,20 @@ public:
             ap.ob[0] = rb[0]; ap.ob[1] = rb[1]; ap.ob[2] = rb[2]; ap.ob[3] = rb[3]; ap.ob[4] = rb[7];
             ap.etapart = w.etap;
             ap.hall = P.hall;
-            DASHA_LAUNCH("a_velocity", 7.0 * N * 8, k_adj_velocity<<<(unsigned)((N + 255) / 256), 256, 0, st>>>(N, mz, g, ap.s, ap.v));
-            DASHA_LAUNCH("a_pointwise", 43.0 * N * 8, k_adj_pointwise<<<(unsigned)w.netap, 128, 0, st>>>(g, ap));
-            DASHA_LAUNCH("a_reduce", 0.0, k_reduce_add<<<1, 1024, 0, st>>>(w.etap, w.netap, w.eta_acc));
+            DASHA_LAUNCH("a_velocity", 7.0 * N * 8, launch(k_adj_velocity, (unsigned)((N + 255) / 256), 256, 0, N, mz, g, ap.s, ap.v));
+            DASHA_LAUNCH("a_pointwise", 43.0 * N * 8, launch(k_adj_pointwise, (unsigned)w.netap, 128, 0, g, ap));
+            DASHA_LAUNCH("a_reduce", 0.0, launch(k_reduce_add, 1, 1024, 0, w.etap, w.netap, w.eta_acc));
             AdjGat ag;
             for (int m = 0; m < 8; ++m) { ag.s.f[m] = Sx[m]; ag.sb.f[m] = sigma[m]; }
             for (int m = 0; m < 4; ++m) ag.wq[m] = w.wq[m];
             for (int m = 0; m < 3; ++m) ag.ub.f[m] = w.ub[m];
             ag.ob[0] = rb[0]; ag.ob[1] = rb[1]; ag.ob[2] = rb[2]; ag.ob[3] = rb[3]; ag.ob[4] = rb[7];
-            DASHA_LAUNCH("a_gather", 25.0 * N * 8, (k_adj_gather<AZG><<<adj_grid(mz, AZG), 128, 0, st>>>(g, ag)));
+            DASHA_LAUNCH("a_gather", 25.0 * N * 8, (launch(k_adj_gather<AZG>, adj_grid(mz, AZG), 128, 0, g, ag)));
             // current chain: 4 transposed avrgc passes, the curl's rows folded, curl^T into B
             T** jt = adj_passes(w.jb, w.jt, w.e0, 3, 4, false, true);
             F3<double> jw, bo;
             for (int m = 0; m < 3; ++m) { jw.f[m] = jt[m]; bo.f[m] = sigma[4 + m]; }
-            DASHA_LAUNCH("a_curlT", 9.0 * N * 8, (k_adj_curlT<AZG><<<adj_grid(mz, AZG), 128, 0, st>>>(g, jw, bo, 1.0, 1)));
+            DASHA_LAUNCH("a_curlT", 9.0 * N * 8, (launch(k_adj_curlT<AZG>, adj_grid(mz, AZG), 128, 0, g, jw, bo, 1.0, 1)));
         }
     }
 
@@ -1589,6 +1593,7 @@ __global__ void k_export_chunk(int mx, int my, int k0, const T* src, const T* co
 // then the current density; one thread per (i, k) on the plane j
 template <class T>
 __global__ void k_midplane(Geo<T> g, int j, F8<T> x, F8<T> comp, F3<T> cur, double* out) {
+    wait_for_stream();
     const int i = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y;
     if (i >= g.mx) return;
     const long n = (long)i + (long)g.mx * (j + (long)g.my * k);

@@ -12,6 +12,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "launch.cuh"
+
 namespace dasha {
 
 constexpr int NF = 8;
@@ -176,6 +178,7 @@ struct FS { T* f[NFLD]; };
 // E = -v x B + eta*J at every node (t3dsdsc.f:1367-1372).
 template <class T>
 __global__ void k_efield(Geo<T> g, F8<T> x, F3<T> cur, F3<T> e) {
+    wait_for_stream();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= g.mx) return;
     int jj = blockIdx.y, k = blockIdx.z;
@@ -193,6 +196,7 @@ __global__ void k_efield(Geo<T> g, F8<T> x, F3<T> cur, F3<T> e) {
 // J0 added to the smoothed J1 (j0_mode FULL).
 template <class T>
 __global__ void k_add_j0(Geo<T> g, F3<T> cur) {
+    wait_for_stream();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= g.mx) return;
     int jj = blockIdx.y, k = blockIdx.z;
@@ -277,6 +281,7 @@ __global__ void __launch_bounds__(256) k_cfl_rate(Geo<T> g, F8<T> x, const doubl
                                                   unsigned long long* next, const unsigned* waits, unsigned long long* late) {
     constexpr int V = 16 / (int)sizeof(T);
     constexpr unsigned ALL = 0xffffffffu;
+    wait_for_stream();
     if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
         *next = 0;                        // the word the next sweep takes
         *late = waits ? *waits : 0;       // ring waits that ran out in the launches before, for the same copy
@@ -392,6 +397,7 @@ template <class T>
 __global__ void __launch_bounds__(128) k_diag_parts(Geo<T> g, F8<T> x, F3<T> cur, const double* wx, const double* wy,
                                                     const double* wz, double gamma, double* part, double* fl, double* jext,
                                                     int klo, int khi, int ka, int kb) {
+    wait_for_stream();
     constexpr int V = 16 / (int)sizeof(T);
     __shared__ double s1[32], s2[32];
     const int tid = threadIdx.x, nj = (g.my + DIAG_J - 1) / DIAG_J;
@@ -465,6 +471,7 @@ __global__ void __launch_bounds__(128) k_diag_parts(Geo<T> g, F8<T> x, F3<T> cur
 // extrema left to one thread and a row's result per (j, k) it took 105 us on 256x128x256, 138 us on 512x256x256.
 static __global__ void __launch_bounds__(1024) k_diag_final(const double* rows, long nrows, const double* fl, int my,
                                                             const double* jext, int mz, double* out, int* blowup) {
+    wait_for_stream();
     __shared__ double sh[3][32], ex[6][32];
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     double sm = 0., se = 0., f = 0.;

@@ -69,6 +69,7 @@ struct NoallocNode {
 
 // J1 = curl(B - B0) with the wall rows (current t3dsdsc.f:2468-2491, bndryc)
 __global__ void __launch_bounds__(128, 8) k_noalloc_curl(const __grid_constant__ Geo<double> g, F3<double> b, F3<double> o) {
+    wait_for_stream();
     const NoallocNode t(g);
     if (!t.on) return;
     const Nbr<double> n(g, t.i, t.j, t.k);
@@ -85,6 +86,7 @@ __global__ void __launch_bounds__(128, 8) k_noalloc_curl(const __grid_constant__
 // from the node coordinates, wall rows re-applied (bndryc t3dsdsc.f:2614-2642).  1/32 + 3/64 (1 + tanh u) =
 // 1/32 + (3/32) / (1 + exp(-2u)), u = (r-3)/3: half the operations of tanh.
 __global__ void __launch_bounds__(128, 8) k_noalloc_smooth(const __grid_constant__ Geo<double> g, F3<double> in, F3<double> out) {
+    wait_for_stream();
     const NoallocNode t(g);
     if (!t.on) return;
     const int im = wrapi(t.i - 1, g.mx) - t.i, ip = wrapi(t.i + 1, g.mx) - t.i;
@@ -111,6 +113,7 @@ __global__ void __launch_bounds__(128, 8) k_noalloc_smooth(const __grid_constant
 // The 1-D tables of axis blockIdx.y from the coordinates x | y | z (`coord`): the first-derivative weights
 // as the derivatives at x0 of the Lagrange polynomials through the five nodes, and the difc weights.
 __global__ void k_noalloc_tables(double* dtab, const double* coord, int mx, int my, int mz) {
+    wait_for_stream();
     const int d = blockIdx.y, n = d == 0 ? mx : (d == 1 ? my : mz), i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     double* t = dtab + (long)d * kTabPerAxis * kAxisMax;
@@ -272,10 +275,10 @@ extern "C" int dasha_current_noalloc(const dasha_grid_c* grid, const double* db_
     }
     const dim3 grd((unsigned)((mx * my + 127) / 128), (unsigned)(mz - 4));
     // J1 = curl(B - B0) with the wall rows, then 4 passes cur -> scratch -> cur -> scratch -> cur
-    k_noalloc_curl<<<grd, 128, 0, st>>>(g, b, cur);
+    launch_overlapped(st, true, k_noalloc_curl, grd, 128, 0, g, b, cur);
     for (int pass = 0; pass < 4; ++pass) {
-        if (pass % 2 == 0) k_noalloc_smooth<<<grd, 128, 0, st>>>(g, cur, tmp);
-        else k_noalloc_smooth<<<grd, 128, 0, st>>>(g, tmp, cur);
+        if (pass % 2 == 0) launch_overlapped(st, true, k_noalloc_smooth, grd, 128, 0, g, cur, tmp);
+        else launch_overlapped(st, true, k_noalloc_smooth, grd, 128, 0, g, tmp, cur);
     }
     return cudaGetLastError() == cudaSuccess ? DASHA_OK : DASHA_E_CUDA;
 }

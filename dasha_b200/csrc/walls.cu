@@ -22,6 +22,7 @@ using walls::Box;
 // (up to 96 registers, the compiler's choice) 4.67.
 template <class F>
 __global__ void __launch_bounds__(128, 8) k_walls(const __grid_constant__ Box b, const __grid_constant__ F f) {
+    wait_for_stream();
     const unsigned nx = (unsigned)(b.x1 - b.x0 + 1), i = blockIdx.x * 128u + threadIdx.x, jy = i / nx;
     if (jy > (unsigned)(b.y1 - b.y0)) return;
     f(b.x0 + (int)(i - jy * nx), b.y0 + (int)jy, b.z0 + (int)blockIdx.y);
@@ -35,7 +36,7 @@ struct GpuExec {
     }
     template <class F>
     void run(Box b, F f) {
-        if (!empty(b)) k_walls<<<grid(b), 128, 0, st>>>(b, f);
+        if (!empty(b)) launch_overlapped(st, true, k_walls<F>, grid(b), 128, 0, b, f);
     }
     // the minimum of positive doubles through their bit patterns (ordered as unsigned integers)
     __host__ __device__ static void atomic_min_bits(unsigned long long* p, double v) {

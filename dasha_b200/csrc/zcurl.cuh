@@ -92,6 +92,7 @@ __global__ void __launch_bounds__(32 * TY) k_zcurl(Geo<T> g, SrcFields<T, 3> src
         }
         cp_async_commit();
     };
+    wait_for_stream();
 #pragma unroll
     for (int p = 0; p < D + 4; ++p) issue(cA - 2 + p);   // planes cA-2 .. cA+1+D
 

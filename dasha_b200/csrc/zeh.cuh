@@ -91,6 +91,7 @@ __global__ void __launch_bounds__(32 * TY) k_zeh(Geo<T> g, EHIO<T> io, int chunk
         }
         cp_async_commit();
     };
+    wait_for_stream();
 #pragma unroll
     for (int p = 0; p < D + 4; ++p) issue(cA - 2 + p);   // planes cA-2 .. cA+1+D
 

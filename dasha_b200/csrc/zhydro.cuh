@@ -168,6 +168,7 @@ __device__ __forceinline__ void zhydro_body(const Geo<T>& g, const HydroIO<T>& i
             }
         }
     };
+    wait_for_stream();
 #pragma unroll
     for (int p = 0; p < D + 4; ++p) issue(cA - 2 + p);   // planes cA-2 .. cA+1+D
 

@@ -190,6 +190,7 @@ __global__ void __launch_bounds__(TX* TYH, MINB) k_zst2(Geo<T> g, SrcFields<T, N
             }
         }
     };
+    wait_for_stream();
 #pragma unroll
     for (int p = 0; p < D + 4; ++p) issue(cA - 2 + p);      // planes cA-2 .. cA+1+D
     const int gi = x0 + tx, gj = y0 + ty;

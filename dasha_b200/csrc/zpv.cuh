@@ -363,6 +363,7 @@ __device__ __forceinline__ void zpv_body(const Geo<T>& g, const SrcFields<T, NF>
         }
         cp_async_commit();
     };
+    wait_for_stream();
 #pragma unroll
     for (int p = 0; p < D + 2; ++p) issue(cA - 1 + p);   // planes cA-1 .. cA+D
 

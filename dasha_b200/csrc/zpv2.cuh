@@ -110,6 +110,7 @@ __global__ void __launch_bounds__(32 * (TY + 2)) k_zpv2(Geo<T> g, SrcFields<T, N
         }
         cp_async_commit();
     };
+    wait_for_stream();
 #pragma unroll
     for (int p = 0; p < D + 2; ++p) issue(pA - 1 + p);   // input planes pA-1 .. pA+D
 
