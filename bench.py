@@ -215,12 +215,13 @@ def run_reference(args, rank, world):
 # the current and E chains both run the 3-field radial-coefficient smoothing pass).
 KERNEL_OF = {
     "k_zpv_J": "k_zpv<3 fields, radial coef, store>", "k_zpv_E": "k_zpv<3 fields, radial coef, store>",
-    "k_zpv_H": "k_zpv2<3 fields, 1/8, two passes>", "k_zpv_EH": "k_zpv<6 fields, E + Hall sum>",
-    "k_zpv_X": "k_zpv<4 fields, store>", "k_zpv_F": "k_zpv<4 fields, store>",
-    "k_zpv_X_rk1": "k_zpv<4 fields, RK stage update>", "k_zpv_X_rk2": "k_zpv<4 fields, RK stage update>",
-    "k_zpv_X_rk3": "k_zpv<4 fields, RK stage update>", "k_zpv_X_rk4": "k_zpv<4 fields, RK stage update>",
-    "k_zpv_F1": "k_zpv<field pairs, compensated filter pass 1>",
-    "k_zpv_F2": "k_zpv<4 fields, compensated filter pass 2>",
+    "k_zpv_H": "k_zpv<3 fields, 1/8, store>", "k_zpv_EH": "k_zpv<6 fields, E + Hall sum>",
+    "k_zpv_E_H": "k_zpv_two<3 fields, E and Hall pass>", "k_zpv_H2": "k_zpv2<3 fields, 1/8, two passes>",
+    "k_zpv_X": "k_zpv_two<4 fields, store>", "k_zpv_F": "k_zpv_two<4 fields, store>",
+    "k_zpv_X_rk1": "k_zpv_two<4 fields, RK stage update>", "k_zpv_X_rk2": "k_zpv_two<4 fields, RK stage update>",
+    "k_zpv_X_rk3": "k_zpv_two<4 fields, RK stage update>", "k_zpv_X_rk4": "k_zpv_two<4 fields, RK stage update>",
+    "k_zpv_F1": "k_zpv_two<field pairs, compensated filter pass 1>",
+    "k_zpv_F2": "k_zpv_two<4 fields, compensated filter pass 2>",
     "k_rhs_hydro": "k_zhydro", "k_efield_hall": "k_zeh", "k_curl": "k_zcurl<+1>",
     "k_rhs_induction": "k_zcurl<-1>", "k_cfl": "k_cfl_rate",
 }
@@ -230,8 +231,8 @@ def kernel_of(tag, prec):
     """The __global__ a tag launches: the smoothing passes and the hydro RHS load their rings by
     TMA (k_zpv_tma, k_zhydro_tma) in FP64, and in FP32 for the passes of 4 and 6 fields."""
     k = KERNEL_OF.get(tag, tag)
-    if k.startswith("k_zpv<") and (prec == "fp64" or not k.startswith("k_zpv<3 ")):
-        return "k_zpv_tma<" + k[len("k_zpv<"):]
+    if k.startswith(("k_zpv<", "k_zpv_two<")) and (prec == "fp64" or "<3 " not in k):
+        return k.replace("<", "_tma<", 1)
     if k == "k_zhydro":
         return "k_zhydro_tma"
     return k

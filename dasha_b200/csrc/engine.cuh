@@ -776,6 +776,45 @@ public:
         return cudaFuncSetAttribute(zpv2_fn<NF, KINDS, Epi>(), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)ZV2c<NF>::smem());
     }
+    // two independent passes of NF fields each in one launch (k_zpv_two)
+    template <int NF, unsigned KA, unsigned KB, class EA, class EB, int MODE>
+    static constexpr auto two_fn() { return k_zpv_two<T, NF, KA, KB, ZVX, ZC<NF>::TYH, ZC<NF>::RY, ZC<NF>::D, EA, EB, MODE>; }
+#ifndef DASHA_NO_TMA
+    template <int NF, unsigned KA, unsigned KB, class EA, class EB, int MODE>
+    static constexpr auto two_tma_fn() { return k_zpv_two_tma<T, NF, KA, KB, ZVX, ZC<NF>::TYH, ZC<NF>::RY, ZC<NF>::D, EA, EB, MODE>; }
+#endif
+    template <int NF, unsigned KA, unsigned KB, int MODE = 0, class EA, class EB>
+    void zp_two(const char* tag, double bytes, const SrcFields<T, NF>& sa, const EA& ea, const SrcFields<T, NF>& sb, const EB& eb) {
+        using Z = ZVc<NF>;
+        dim3 gg((mx + Z::TX - 1) / Z::TX, (my + Z::TY - 1) / Z::TY, 1);
+        const int tiles = 2 * (int)(gg.x * gg.y);
+#ifndef DASHA_NO_TMA
+        if constexpr (zp_tma<NF>()) {
+            const auto fn = two_tma_fn<NF, KA, KB, EA, EB, MODE>();
+            const int ch = zchunk(tiles, (const void*)fn, 32 * ZC<NF>::TYH, Z::smem_tma()), nz = (mz + ch - 1) / ch;
+            gg.z = 2 * nz;
+            ZpMaps ma, mb;
+            if (!zpv_maps<NF>(sa, ma) || !zpv_maps<NF>(sb, mb)) launch_err = "cuTensorMapEncodeTiled failed for a smoothing pass";
+            DASHA_LAUNCH(tag, bytes, launch(fn, gg, 32 * ZC<NF>::TYH, Z::smem_tma(), g, sa, ea, sb, eb, ch, nz, ma, mb));
+        } else
+#endif
+        {
+            const auto fn = two_fn<NF, KA, KB, EA, EB, MODE>();
+            const int ch = zchunk(tiles, (const void*)fn, 32 * ZC<NF>::TYH, Z::smem()), nz = (mz + ch - 1) / ch;
+            gg.z = 2 * nz;
+            DASHA_LAUNCH(tag, bytes, launch(fn, gg, 32 * ZC<NF>::TYH, Z::smem(), g, sa, ea, sb, eb, ch, nz));
+        }
+    }
+    template <int NF, unsigned KA, unsigned KB, class EA, class EB, int MODE = 0>
+    static cudaError_t two_attr() {
+#ifndef DASHA_NO_TMA
+        if constexpr (zp_tma<NF>())
+            return cudaFuncSetAttribute(two_tma_fn<NF, KA, KB, EA, EB, MODE>(), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)ZVc<NF>::smem_tma());
+#endif
+        return cudaFuncSetAttribute(two_fn<NF, KA, KB, EA, EB, MODE>(), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)ZVc<NF>::smem());
+    }
     // k_zcurl: tile 32*ZVX x 8, one row per warp, 2 planes in flight beyond c+2
     using ZC3c = ZC3<T, ZVX, 8, 2>;
     template <int SIGN>
@@ -819,25 +858,23 @@ public:
     using ZEHc = ZEH<T, ZVX, 8, 2>;   // k_zeh: tile 32*ZVX x 8, 2 planes in flight beyond c+2
     using St3 = VStore<T, 3, ZVX>;
     using St4 = VStore<T, 4, ZVX>;
-    using Acc3 = VAcc<T, 3, ZVX>;
     using RK4 = VRK<T, 4, ZVX, KAHAN>;
     cudaError_t zs_attr() {
         cudaError_t e;
         if ((e = zp_attr1<3, 0u, St3>())) return e;
         if ((e = zp_attr1<3, KIND_H, St3>())) return e;
-        if ((e = zp_attr1<3, KIND_H, Acc3>())) return e;
         if ((e = zp_attr1<6, KIND_EH, VSum<T, 3, ZVX>>())) return e;
-        if ((e = zp_attr1<4, 0u, St4>())) return e;
-        if ((e = zp_attr1<4, KIND_B4, St4>())) return e;
-        if ((e = zp_attr1<4, 0u, RK4>())) return e;
-        if ((e = zp_attr1<4, KIND_B4, RK4>())) return e;
-        if ((e = zp2_attr1<3, KIND_H, St3>())) return e;
+        if ((e = two_attr<3, 0u, KIND_H, St3, St3>())) return e;
+        if constexpr (KAHAN)
+            if ((e = zp2_attr1<3, KIND_H, St3>())) return e;
+        if ((e = two_attr<4, 0u, KIND_B4, St4, St4>())) return e;
+        if ((e = two_attr<4, 0u, KIND_B4, RK4, RK4>())) return e;
         if constexpr (KAHAN) {
-            if ((e = zp_attr1<4, 0u, VStore<T, 2, ZVX>, 1>())) return e;
-            if ((e = zp_attr1<4, KIND_P45, VStore<T, 2, ZVX>, 1>())) return e;
-            if ((e = zp_attr1<4, KIND_P67, VStore<T, 2, ZVX>, 1>())) return e;
-            if ((e = zp_attr1<4, 0u, VKF<T, 4, ZVX>, 2>())) return e;
-            if ((e = zp_attr1<4, KIND_B4, VKF<T, 4, ZVX>, 2>())) return e;
+            using Inc = VStore<T, 2, ZVX>;
+            using Kah = VKF<T, 4, ZVX>;
+            if ((e = two_attr<4, 0u, 0u, Inc, Inc, 1>())) return e;
+            if ((e = two_attr<4, KIND_P45, KIND_P67, Inc, Inc, 1>())) return e;
+            if ((e = two_attr<4, 0u, KIND_B4, Kah, Kah, 2>())) return e;
         }
         if ((e = cudaFuncSetAttribute(k_zst2<T, 5, ZTX, 8, HMINB, OpHydro<T>>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)ZS2<T, 5, ZTX, 8>::smem(true))))
@@ -864,14 +901,13 @@ public:
     static constexpr unsigned KIND_EH = (1u << 6) | (1u << 8) | (1u << 10);         // E (radial) then Hall (1/8)
     static constexpr unsigned KIND_P67 = 2u;                                        // field pair (B3, p)
 
-    // one avrg/avrgtt pass over the 8 state-like fields, as two 4-field launches (rho, m) and
-    // (B, p); mk(lo) builds the epilogue of fields lo..lo+3
+    // one avrg/avrgtt pass over the 8 state-like fields, (rho, m) and (B, p) by 4 fields in one
+    // launch; mk(lo) builds the epilogue of fields lo..lo+3
     template <class MkEpi>
     void pass8(const char* tag, double bytes_per_cell, T* const* in, MkEpi mk) {
         SrcFields<T, 4> a, b;
         for (int q = 0; q < 4; ++q) { a.f[q] = in[q]; b.f[q] = in[4 + q]; }
-        zp<4, 0u>(tag, 0.5 * bytes_per_cell * N * sizeof(T), a, mk(0));
-        zp<4, KIND_B4>(tag, 0.5 * bytes_per_cell * N * sizeof(T), b, mk(4));
+        zp_two<4, 0u, KIND_B4>(tag, bytes_per_cell * N * sizeof(T), a, mk(0), b, mk(4));
     }
     static St4 st4(T* const* p, int lo) { St4 s; for (int q = 0; q < 4; ++q) s.f[q] = p[lo + q]; return s; }
     // values per field the RK stage epilogue reads and writes (base, acc, x, comp)
@@ -906,23 +942,24 @@ public:
     // avrgtt on the compensated FP32 state (X, C): pass 1 writes its increment of X - C into
     // t, pass 2 adds the two-pass increment to (X, C) in place with a Kahan step
     void filter_compensated(T* const* t) {
-        for (int lo = 0; lo < 8; lo += 2) {   // pass 1 by field pairs: ring (x_a, x_b, comp_a, comp_b)
-            SrcFields<T, 4> a;
-            VStore<T, 2, ZVX> o;
-            for (int q = 0; q < 2; ++q) { a.f[q] = X[lo + q]; a.f[2 + q] = C[lo + q]; o.f[q] = t[lo + q]; }
-            const double by = 6.0 * N * sizeof(T);
-            if (lo < 4) zp<4, 0u, 1>("k_zpv_F1", by, a, o);
-            else if (lo == 4) zp<4, KIND_P45, 1>("k_zpv_F1", by, a, o);
-            else zp<4, KIND_P67, 1>("k_zpv_F1", by, a, o);
-        }
+        // pass 1 by field pairs: ring (x_a, x_b, comp_a, comp_b), two pairs a launch
+        SrcFields<T, 4> a[4], d[2];
+        VStore<T, 2, ZVX> o[4];
+        VKF<T, 4, ZVX> e[2];
+        for (int m = 0; m < 4; ++m)
+            for (int q = 0; q < 2; ++q) {
+                a[m].f[q] = X[2 * m + q]; a[m].f[2 + q] = C[2 * m + q];
+                o[m].f[q] = t[2 * m + q];
+            }
+        zp_two<4, 0u, 0u, 1>("k_zpv_F1", 12.0 * N * sizeof(T), a[0], o[0], a[1], o[1]);
+        zp_two<4, KIND_P45, KIND_P67, 1>("k_zpv_F1", 12.0 * N * sizeof(T), a[2], o[2], a[3], o[3]);
         hx(t, 8);
-        for (int lo = 0; lo < 8; lo += 4) {
-            SrcFields<T, 4> d;
-            VKF<T, 4, ZVX> e;
-            for (int q = 0; q < 4; ++q) { d.f[q] = t[lo + q]; e.x[q] = X[lo + q]; e.comp[q] = C[lo + q]; }
-            if (lo == 0) zp<4, 0u, 2>("k_zpv_F2", 20.0 * N * sizeof(T), d, e);
-            else zp<4, KIND_B4, 2>("k_zpv_F2", 20.0 * N * sizeof(T), d, e);
-        }
+        for (int m = 0; m < 2; ++m)
+            for (int q = 0; q < 4; ++q) {
+                d[m].f[q] = t[4 * m + q];
+                e[m].x[q] = X[4 * m + q]; e[m].comp[q] = C[4 * m + q];
+            }
+        zp_two<4, 0u, KIND_B4, 2>("k_zpv_F2", 40.0 * N * sizeof(T), d[0], e[0], d[1], e[1]);
     }
 
     T** curF = nullptr;   // smoothed current after launch_current
@@ -931,28 +968,9 @@ public:
     // n smoothing passes of 3 fields, ping-pong between a and b starting from a; returns the
     // buffer holding the result.  On a z-slab every pass output that a later pass reads has its
     // ghost planes refreshed, the last one too when xlast (a later launch reads it at
-    // z-neighbours), and the Hall pairs run as single passes: k_zpv2 forms its first pass on the
-    // planes next to the slab ends from the wall rule.  Both give the same values: the fused
-    // pair rounds as two single passes.
-    // Pass pairs of the Hall chain (constant coefficient 1/8) run fused in k_zpv2.  Measured on
-    // B200 (FP32 1024x512x1024 / FP64 512x256x512 step): Hall pairs fused 436.0 / 107.7 ms,
-    // nothing fused 442.1 / 108.4; fusing the radial-coefficient chains J and E as well 437.3 /
-    // 186.7 with everything; the xdif pair with the RK update 138.4 (FP64), the FP64 filter
-    // 114.1: where the coefficient is evaluated per node, or the epilogue is heavy, the doubled
-    // per-node work and the lower occupancy of the 320-thread CTA outweigh the saved traffic.
+    // z-neighbours).
     template <unsigned KINDS>
     T** passes3(const char* tag, T** a, T** b, int n, bool xlast) {
-        if constexpr (KINDS == KIND_H) {
-            if (!cut()) {
-                for (int p = 0; p < n; p += 2) {   // pairs of passes in one k_zpv2 launch, a lone last one by k_zpv
-                    T** in = ((p / 2) & 1) ? b : a;
-                    T** out = ((p / 2) & 1) ? a : b;
-                    if (p + 1 < n) zp2<3, KINDS>(tag, 6.0 * N * sizeof(T), src3(in), st3(out));
-                    else zp<3, KINDS>(tag, 6.0 * N * sizeof(T), src3(in), st3(out));
-                }
-                return (((n + 1) / 2) & 1) ? b : a;
-            }
-        }
         for (int p = 0; p < n; ++p) {
             T** in = (p & 1) ? b : a;
             T** out = (p & 1) ? a : b;
@@ -961,6 +979,13 @@ public:
         }
         return (n & 1) ? b : a;
     }
+    // The Hall chain's passes 1-4 as two fused pairs (k_zpv2), or one by one with the E chain's passes (k_zpv_two)?  Pairs save
+    // a read and a write of the fields, passes the halo and level-1 work of 320-thread CTAs: on large planes, where memory
+    // sets the pace, pairs win (1024x512x512 FP32 181.2 against 182.7 ms a step), on 512x256 planes and below the
+    // passes do (512x256x256 FP32 22.64 against 22.85, 512x256x512 FP64 86.4 against 88.0, 64x32x64 FP32 0.289
+    // against 0.339); FP64, whose passes are longer, at every size measured.  Both give the same values: a pair rounds as
+    // two single passes.  A z-slab takes the passes: k_zpv2 forms its first pass next to the slab ends from the wall rule.
+    bool hall_pairs() const { return KAHAN && !cut() && (long)mx * my > 262144; }
 
     // smoothed current of state xs (current, t3dsdsc.f:2452-2500): curl, 4 passes
     const char* launch_err = nullptr;   // a launch that could not be set up (reported by stepon)
@@ -1034,10 +1059,30 @@ public:
         }
         hx(E[0], 3);
         if (P.hall) {
-            // avrgh passes 1-4, avrgE passes 1-3, then one 6-field launch: the 4th E pass and the
+            // avrgh passes 1-4 and avrgE passes 1-3, then one 6-field launch: the 4th E pass and the
             // 5th Hall pass, summed into E (the two chains are independent until that sum)
-            T** h = passes3<KIND_H>("k_zpv_H", Hh[0], Hh[1], 4, true);
-            T** e3 = passes3<0u>("k_zpv_E", E[0], cother, 3, true);
+            T** h = Hh[0];
+            T** e3 = E[0];
+            bool pairs = false;
+            if constexpr (KAHAN) pairs = hall_pairs();
+            if (pairs) {
+                if constexpr (KAHAN) {
+                    zp2<3, KIND_H>("k_zpv_H2", 6.0 * N * sizeof(T), src3(Hh[0]), st3(Hh[1]));
+                    zp2<3, KIND_H>("k_zpv_H2", 6.0 * N * sizeof(T), src3(Hh[1]), st3(Hh[0]));
+                }
+                e3 = passes3<0u>("k_zpv_E", E[0], cother, 3, true);
+            } else {
+                h = passes3<KIND_H>("k_zpv_H", Hh[0], Hh[1], 1, true);
+                for (int p = 0; p < 3; ++p) {
+                    T** ho = h == Hh[0] ? Hh[1] : Hh[0];
+                    T** eo = e3 == E[0] ? cother : E[0];
+                    zp_two<3, 0u, KIND_H>("k_zpv_E_H", 12.0 * N * sizeof(T), src3(e3), st3(eo), src3(h), st3(ho));
+                    e3 = eo;
+                    h = ho;
+                    hx(e3, 3);
+                    hx(h, 3);
+                }
+            }
             T** eo = e3 == E[0] ? cother : E[0];
             SrcFields<T, 6> se;
             VSum<T, 3, ZVX> es;
@@ -1099,7 +1144,7 @@ public:
         (void)time;
         NvtxRange range("stepon");
         // stages 1..4: base = X, stage state in S, accumulator in A; both xdif smoothing
-        // passes run in one k_zpv2 launch per field pair that ends in the RK stage update.
+        // passes of all 8 fields are one launch each, the second ends in the RK stage update.
         const int every = P.filter_every > 0 ? P.filter_every : 1;
         const bool filt = nstep % every == 0;
         hx(X, 8);
@@ -1118,10 +1163,7 @@ public:
             } else {
                 pass8("k_zpv_F", 16.0, X, [&](int lo) { return st4(t, lo); });
                 hx(t, 8);
-                SrcFields<T, 4> a, b;
-                for (int q = 0; q < 4; ++q) { a.f[q] = t[q]; b.f[q] = t[4 + q]; }
-                zp<4, 0u>("k_zpv_F", 8.0 * N * sizeof(T), a, st4(S, 0));
-                zp<4, KIND_B4>("k_zpv_F", 8.0 * N * sizeof(T), b, st4(S, 4));
+                pass8("k_zpv_F", 16.0, t, [&](int lo) { return st4(S, lo); });
                 for (int m = 0; m < 8; ++m) std::swap(X[m], S[m]);
             }
         }

@@ -3,7 +3,7 @@
 // shared-memory ring filled by cp.async.  Global memory is read once per plane (plus the x-y
 // halo, which neighbouring CTAs read at about the same time and so mostly hits L2) and
 // written once.  This file holds the shared helpers and the radius-2 ring framework k_zst2
-// (hydro RHS); the smoothing passes are k_zpv / k_zpv2 (zpv.cuh, zpv2.cuh), the curls k_zcurl
+// (hydro RHS); the smoothing passes are k_zpv / k_zpv_two / k_zpv2 (zpv.cuh, zpv2.cuh), the curls k_zcurl
 // (zcurl.cuh).
 #pragma once
 #include "mhd_kernels.cuh"
