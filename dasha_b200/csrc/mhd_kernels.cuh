@@ -121,53 +121,7 @@ struct Nbr {
         return d1fc(f[c - 2 * g.sz], f[c - g.sz], f[c], f[c + g.sz], f[c + 2 * g.sz],
                     g.a1z[k], g.b1z[k], g.c1z[k], g.d1z[k]);
     }
-    __device__ __forceinline__ T D2x(const Geo<T>& g, const T* f) const {
-        return d1fc(f[xm2], f[xm1], f[c], f[xp1], f[xp2], g.a2x[i], g.b2x[i], g.c2x[i], g.d2x[i]);
-    }
-    __device__ __forceinline__ T D2y(const Geo<T>& g, const T* f) const {
-        return d1fc(f[ym2], f[ym1], f[c], f[yp1], f[yp2], g.a2y[j], g.b2y[j], g.c2y[j], g.d2y[j]);
-    }
-    __device__ __forceinline__ T D2z(const Geo<T>& g, const T* f) const {
-        return d1fc(f[c - 2 * g.sz], f[c - g.sz], f[c], f[c + g.sz], f[c + 2 * g.sz],
-                    g.a2z[k], g.b2z[k], g.c2z[k], g.d2z[k]);
-    }
-    // one Jacobi smoothing stencil: difc_x + difc_y + difc_z (t3dsdsc.f:5643-5648)
-    __device__ __forceinline__ T difc3(const Geo<T>& g, const T* f) const {
-        T f0 = f[c];
-        T tx = (f[xp1] - f0) * g.wpx[i] - (f0 - f[xm1]) * g.wmx[i];
-        T ty = (f[yp1] - f0) * g.wpy[j] - (f0 - f[ym1]) * g.wmy[j];
-        T tz = (f[c + g.sz] - f0) * g.wpz[k] - (f0 - f[c - g.sz]) * g.wmz[k];
-        return tx + ty + tz;
-    }
 };
-
-// Row rule of the z walls: which interior row a wall row copies from, and the factor.
-__device__ __forceinline__ int wall_src(int k, int mz, bool& zero, bool& half) {
-    zero = (k == 0 || k == mz - 1);
-    half = (k == 1 || k == mz - 2);
-    if (k == 1) return 2;
-    if (k == mz - 2) return mz - 3;
-    return k;
-}
-
-// ---------------------------------------------------------------------------------------
-// J1 = curl(B - B0) on interior rows + wall rows (current t3dsdsc.f:2468-2491, bndryc).
-template <class T>
-__global__ void k_curl(Geo<T> g, F3<T> b, F3<T> j) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= g.mx) return;
-    int jj = blockIdx.y, k = blockIdx.z;
-    bool zero, half;
-    int ks = wall_src(k, g.mz, zero, half);
-    long c = (long)i + (long)jj * g.sy + (long)k * g.sz;
-    if (zero) { j.f[0][c] = T(0); j.f[1][c] = T(0); j.f[2][c] = T(0); return; }
-    Nbr<T> n(g, i, jj, ks);
-    T cx = n.Dy(g, b.f[2]) - n.Dz(g, b.f[1]);
-    T cy = n.Dz(g, b.f[0]) - n.Dx(g, b.f[2]);
-    T cz = n.Dx(g, b.f[1]) - n.Dy(g, b.f[0]);
-    if (half) { cx = T(0.5) * cx; cy = T(0.5) * cy; cz = T(0.5) * cz; }
-    j.f[0][c] = cx; j.f[1][c] = cy; j.f[2][c] = cz;
-}
 
 // ---------------------------------------------------------------------------------------
 // NFLD field pointers (the transposed smoothing passes of the adjoint)
