@@ -915,10 +915,6 @@ public:
     // both xdif avrg passes of the raw RHS k, the second ending in the RK stage update: x =
     // stage state (or the step result at stage 4), base, acc, comp (FP32 Kahan compensation or
     // null)
-
-    // both xdif avrg passes of the raw RHS k, the second ending in the RK stage update: x =
-    // stage state (or the step result at stage 4), base, acc, comp (FP32 Kahan compensation or
-    // null)
     void rk_passes(int stage, double dt, T* const* k, T* const* base, T* const* x, T* const* acc, T* const* comp) {
         static const char* names[4] = {"k_zpv_X_rk1", "k_zpv_X_rk2", "k_zpv_X_rk3", "k_zpv_X_rk4"};
         T* t[8];
