@@ -200,7 +200,10 @@ public:
     // the equilibrium, then xresd as initia computes it (T:805-834): the state set to the
     // equilibrium, right(0, 1e-9, 1) with eta = 0 (foreta runs after it), xresd = the momentum rates
     Status equilibrium_from(const double* src, long ld1, long ld2) {
-        Status s = upload(src, ld1, ld2, 5, a.xm, a.xdif);   // rho0 bx0 by0 bz0 p0 by way of xm
+        // rho0 bx0 by0 bz0 p0 by way of xm, zero off the physical nodes: the driver reads rhoi beyond the last
+        // plane where mz - 1 >= 3 my (RowRule::driven_state), and rhs() packs its rates in xm
+        DASHA_CK(cudaMemsetAsync(a.xm, 0, sizeof(double) * 5 * n, st));
+        Status s = upload(src, ld1, ld2, 5, a.xm, a.xdif);
         if (s.code) return s;
         double* eq[5] = {a.rhoi, a.bxi, a.byi, a.bzi, a.pri};
         for (int q = 0; q < 5; ++q) DASHA_CK(cudaMemcpyAsync(eq[q], a.xm + q * n, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
