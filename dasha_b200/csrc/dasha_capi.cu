@@ -131,15 +131,14 @@ static int bounds_status(dasha_ctx* c, int rc) {
 static int bounds_status(dasha_ctx*, int rc) { return rc; }
 #endif
 #ifndef DASHA_NO_TMA
-// a bounded mbarrier wait of a TMA ring that ran out (the kernel returned early)
+// a bounded mbarrier wait of a TMA ring that ran out in a launch of this context (the kernel returned early).  The word is
+// the context's and stays set: its state lacks a pass, and the failure is sticky
 static int wait_status(dasha_ctx* c, int rc) {
     if (!c || !c->st) return rc;
+    if (cudaStreamSynchronize(c->st) != cudaSuccess) return rc;
+    const unsigned* word = c->eng ? c->eng->ring_late() : nullptr;
     unsigned int hit = 0;
-    if (cudaStreamSynchronize(c->st) != cudaSuccess || cudaMemcpyFromSymbol(&hit, g_wait_timeout, sizeof(hit)) != cudaSuccess)
-        return rc;
-    if (!hit) return rc;
-    const unsigned int zero = 0;
-    cudaMemcpyToSymbol(g_wait_timeout, &zero, sizeof(zero));
+    if (!word || cudaMemcpy(&hit, word, sizeof(hit), cudaMemcpyDeviceToHost) != cudaSuccess || !hit) return rc;
     return fail(c, DASHA_E_CUDA, RING_WAIT_MSG);
 }
 #else
@@ -690,6 +689,15 @@ int dasha_adjoint_rhs(dasha_ctx* c, const double* w_f, double* out_f, long ld1, 
     if (!c->state_set) return fail(c, DASHA_E_STATE, "no state set");
     return engine_call(c, [&] { return c->eng->adjoint_rhs(w_f, out_f, ld1, ld2); });
 }
+
+#ifdef DASHA_BOUNDS
+// the checking build: what a ring wait that ran out in a launch enqueued so far leaves behind
+int dasha_check_ring_wait(dasha_ctx* c) {
+    CAPI_GUARD(c);
+    unsigned* word = c->eng->ring_late();
+    return word && cudaMemsetAsync(word, 1, 1, c->st) == cudaSuccess ? DASHA_OK : DASHA_E_CUDA;
+}
+#endif
 
 int dasha_timer(dasha_ctx* c, int op, double* ms) {
     CAPI_GUARD(c);

@@ -91,6 +91,8 @@ struct EngineBase {
     virtual void set_cfl_k0(int) {}
     // setdt reports the ring waits that ran out (with its rate), and stepon leaves them to the next call that waits
     virtual bool own_wait_status() const { return false; }
+    // the context's word for them on the device (null: no kernel of the engine has rings)
+    virtual unsigned* ring_late() { return nullptr; }
     virtual ~EngineBase() {
         if (t0) cudaEventDestroy(t0);
         if (t1) cudaEventDestroy(t1);
@@ -199,10 +201,9 @@ public:
     double* red = nullptr;       // reduction scratch
     double* cfltab = nullptr;    // CFL rate tables: ich[mx+my+mz], vv[..], ih[..]
     // bits of setdt's largest rate, two words taken in turn (a sweep clears the other one), then the
-    // blow-up flag, then whether a ring wait ran out: one copy reads all
+    // blow-up flag, then whether a ring wait of this context ran out (g.late): one copy reads all
     unsigned long long* rate_bits = nullptr;
     int rate_word = 0;
-    unsigned* waits = nullptr;   // g_wait_timeout
     int* flag = nullptr;         // blow-up flag
     double* hpin = nullptr;      // pinned host scratch
     double* mpd = nullptr;       // the 11 mid-plane output fields (allocated on first use)
@@ -225,6 +226,7 @@ public:
     }
     void set_cfl_k0(int k0) override { g.kcfl0 = k0; }
     bool own_wait_status() const override { return !halo; }
+    unsigned* ring_late() override { return g.late; }
     // a z-slab with a neighbour: its ghost planes are copies (a lone slab's are the walls)
     bool cut() const { return halo && (halo->geo.lower() || halo->geo.upper()); }
     // z-slab contexts: refresh the ghost planes of fields f that a later launch reads at
@@ -358,10 +360,7 @@ public:
         DASHA_CK(cudaMalloc(&rate_bits, 32));
         DASHA_CK(cudaMemsetAsync(rate_bits, 0, 32, st));
         flag = (int*)(rate_bits + 2);
-#ifndef DASHA_NO_TMA
-        DASHA_CK(cudaGetSymbolAddress((void**)&waits, g_wait_timeout));
-#endif
-        DASHA_CK(cudaMemsetAsync(flag, 0, sizeof(int), st));
+        g.late = (unsigned*)(rate_bits + 3);
         DASHA_CK(cudaMallocHost(&hpin, sizeof(double) * 16));
 
         blk = dim3(std::min(128, ((mx + 31) / 32) * 32));
@@ -1236,16 +1235,13 @@ public:
         DASHA_LAUNCH("k_cfl", 8.0 * N * sizeof(T),
                      launch(k_cfl_rate<T>, dim3(bx, (nk + planes - 1) / planes), 256, 0, g, f8(X), cfltab, cfltab + nt, cfltab + 2 * nt, P.gamma,
                          (P.dt_whistler && P.hall) ? P.di * 3.141592653589793 : 0.0, planes, rate_bits + word,
-                         rate_bits + (word ^ 1), waits, rate_bits + 3));
+                         rate_bits + (word ^ 1)));
         DASHA_CK(cudaGetLastError());
         DASHA_CK(cudaMemcpyAsync(hpin + 12, rate_bits, 32, cudaMemcpyDeviceToHost, st));
         DASHA_CK(cudaStreamSynchronize(st));
         unsigned late = 0;
         std::memcpy(&late, hpin + 15, sizeof(late));
-        if (late) {
-            cudaMemset(waits, 0, sizeof(late));
-            return Status::err(DASHA_E_CUDA, RING_WAIT_MSG);
-        }
+        if (late) return Status::err(DASHA_E_CUDA, RING_WAIT_MSG);
         const double v = hpin[12 + word];
         *dt = (v != v) ? v : std::fmin(100.0, 1.0 / v);
         std::memcpy(blowup, hpin + 14, sizeof(int));

@@ -29,6 +29,7 @@ struct Geo {
     // difc weights: difc = (f+ - f0)*wp - (f0 - f-)*wm  (t3dsdsc.f:5618-5619)
     const T *wpx, *wmx, *wpy, *wmy, *wpz, *wmz;
     const T *cbx;    // (1/32)(1 - tanh((x+3)/8)), smoothing coefficient of B (t3dsdsc.f:5636-5642)
+    unsigned* late;  // set by a launch of the context whose bounded ring wait ran out
     const T* cr;     // FP64 contexts: the radial coefficient below at every node, made once (k_radial_field)
     const T *xc, *yc, *zc;   // node coordinates: the radial coefficient 1/32 + 3/32 (1 + tanh((r-3)/3))/2
                              // (t3dsdsc.f:5659-5661); FP32 passes evaluate it per node
@@ -232,14 +233,11 @@ __device__ __forceinline__ void load16(const double* p, double (&v)[2]) {
 template <class T>
 __global__ void __launch_bounds__(256) k_cfl_rate(Geo<T> g, F8<T> x, const double* ich, const double* vv, const double* ih,
                                                   double gamma, double whistler, int planes, unsigned long long* out,
-                                                  unsigned long long* next, const unsigned* waits, unsigned long long* late) {
+                                                  unsigned long long* next) {
     constexpr int V = 16 / (int)sizeof(T);
     constexpr unsigned ALL = 0xffffffffu;
     wait_for_stream();
-    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
-        *next = 0;                        // the word the next sweep takes
-        *late = waits ? *waits : 0;       // ring waits that ran out in the launches before, for the same copy
-    }
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *next = 0;   // the word the next sweep takes
     const int nq = g.mx / V, id = blockIdx.x * blockDim.x + threadIdx.x;
     const bool on = id < nq * (g.my - 1);
     const int jj = on ? id / nq : 0, i0 = on ? V * (id - jj * nq) : 0;

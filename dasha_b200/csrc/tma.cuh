@@ -1,6 +1,6 @@
 // tma.cuh -- ring planes of the z-marching kernels loaded by `cp.async.bulk.tensor` against one
-// mbarrier per ring stage, with waits that give up after about a second (g_wait_timeout,
-// reported by the C-ABI) instead of spinning.  Built unless -DDASHA_NO_TMA (the comparison build
+// mbarrier per ring stage, with waits that give up after about a second (recorded in Geo::late, the context's
+// own word, and reported by its next call that waits) instead of spinning.  Built unless -DDASHA_NO_TMA (the comparison build
 // whose rings all use cp.async).
 #pragma once
 
@@ -11,7 +11,6 @@ namespace dasha {
 __device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 
 #ifndef DASHA_NO_TMA
-static __device__ unsigned int g_wait_timeout;    // a bounded mbarrier wait ran out
 __device__ __forceinline__ void mbar_init(unsigned long long* bar, unsigned count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count) : "memory");
 }

@@ -21,7 +21,7 @@
 // rows y0-2 .. y0+TY+1) lies inside the grid loads each ring plane as 5 `cp.async.bulk.tensor`
 // boxes of exactly the ring plane's layout, issued by thread 0 against one mbarrier per stage;
 // every thread waits on the stage's mbarrier (time-bounded: after about a second the kernel
-// records g_wait_timeout, waits, again bounded, for the boxes it issued and returns) and turns
+// sets Geo::late, waits, again bounded, for the boxes it issued and returns) and turns
 // its share of the plane's rho - rho0 into 1/rho before the plane's barrier.  CTAs whose halo
 // wraps around x or y keep the cp.async element copies (a box cannot wrap).  The compute is the
 // same code in both kernels; the engine picks one.
@@ -223,7 +223,7 @@ __device__ __forceinline__ void zhydro_body(const Geo<T>& g, const HydroIO<T>& i
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             if (__syncthreads_or(late)) {
                 // every box issued so far (planes up to c+2+D) lands before the CTA leaves
-                if (tid == 0) atomicExch(&g_wait_timeout, 1u);
+                if (tid == 0) atomicExch(g.late, 1u);
                 for (int p = c - 2; p <= min(c + 2 + D, phi); ++p) {
                     if (p < cA - 2) continue;
                     mbar_wait_bounded(bars + p % NS, (unsigned)(((p - (cA - 2)) / NS) & 1));

@@ -386,7 +386,7 @@ __device__ __forceinline__ void zpv_body(const Geo<T>& g, const SrcFields<T, NF>
                 if (!mbar_wait_bounded(bars + p % NS, (unsigned)(((p - (cA - 1)) / NS) & 1))) { late = true; break; }
             if (__syncthreads_or(late)) {
                 // every box issued so far (planes up to c+1+D) lands before the CTA leaves
-                if (tid == 0) atomicExch(&g_wait_timeout, 1u);
+                if (tid == 0) atomicExch(g.late, 1u);
                 for (int p = c - 1; p <= min(c + 1 + D, phi); ++p)
                     if (p >= cA - 1) mbar_wait_bounded(bars + p % NS, (unsigned)(((p - (cA - 1)) / NS) & 1));
                 return;

@@ -169,7 +169,8 @@ int dasha_setdt(dasha_ctx* ctx, double time, double* dt_out);
 
 /* One RK4 step (stepon, t3dsdsc.f:1063-1185), enqueued asynchronously.  nstep is the step
  * counter before the step: the post-step filter runs when nstep % filter_every == 0 and the
- * blow-up guard (diagn) when nstep % 10 == 0. */
+ * blow-up guard (diagn) when nstep % 10 == 0.  A step that fails on the GPU is reported by the next call of the
+ * same context that waits for it (dasha_setdt, dasha_get_state, ...), as DASHA_E_CUDA. */
 int dasha_stepon(dasha_ctx* ctx, double time, double dt, int nstep);
 
 /* Smoothed current density cur(mxpr,my,mzpr,3) of the current state (current,
