@@ -135,7 +135,7 @@ static int bounds_status(dasha_ctx*, int rc) { return rc; }
 // the context's and stays set: its state lacks a pass, and the failure is sticky
 static int wait_status(dasha_ctx* c, int rc) {
     if (!c || !c->st) return rc;
-    if (cudaStreamSynchronize(c->st) != cudaSuccess) return rc;
+    if (const cudaError_t e = cudaStreamSynchronize(c->st)) return rc ? rc : fail(c, DASHA_E_CUDA, cudaGetErrorString(e));
     const unsigned* word = c->eng ? c->eng->ring_late() : nullptr;
     unsigned int hit = 0;
     if (!word || cudaMemcpy(&hit, word, sizeof(hit), cudaMemcpyDeviceToHost) != cudaSuccess || !hit) return rc;
@@ -435,6 +435,8 @@ int dasha_checkpoint(dasha_ctx* c, const char* path, int ncase, int nstep, doubl
     SLAB_UNSUPPORTED(c, "dasha_checkpoint");
     if (!path || max_subrecord < 0) return fail(c, DASHA_E_INVALID, "bad checkpoint arguments");
     if (!c->state_set) return fail(c, DASHA_E_STATE, "no state set");
+    // steps enqueued before: one that failed leaves the file at `path` as it is
+    if (int rc = wait_status(c, DASHA_OK)) return rc;
     return host_call(c, [&]() -> int {
         const long maxsub = max_subrecord == 0 ? kMaxSubrecord : std::min(max_subrecord, kMaxSubrecord);
         File f(path, "wb");
@@ -565,6 +567,7 @@ int dasha_m3d_write_ctx(dasha_ctx* c, const char* path, double time) {
     SLAB_UNSUPPORTED(c, "dasha_m3d_write_ctx");
     if (!path) return fail(c, DASHA_E_INVALID, "null path");
     if (!c->state_set) return fail(c, DASHA_E_STATE, "no state set");
+    if (int rc = wait_status(c, DASHA_OK)) return rc;   // as dasha_checkpoint
     return host_call(c, [&]() -> int {
         File f(path, "w");
         if (!f.f) return fail(c, DASHA_E_INVALID, std::string("cannot open ") + path);

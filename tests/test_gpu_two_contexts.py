@@ -67,3 +67,26 @@ def test_a_ring_wait_is_reported_by_its_own_context(call, precision):
     b.stepon(0.0, dt, 1)
     assert np.isfinite(b.get_state()).all()
     b.close()
+
+
+@pytest.mark.parametrize("write", ["checkpoint", "m3d"])
+def test_a_failed_step_leaves_the_files_before_it(write, tmp_path):
+    """dasha_checkpoint and dasha_m3d_write_ctx look for the step's status before they open their file: the last good
+    one stays as it is."""
+    lib = capi.bind(capi.BOUNDS_LIB_PATH)
+    lib.dasha_check_ring_wait.argtypes = [C.c_void_p]
+    d = capi.gem_context(CFGS[0], 0, lib=lib)
+    path = str(tmp_path / "file").encode()
+
+    def out():
+        if write == "checkpoint":
+            return lib.dasha_checkpoint(d.h, path, 1, 2, 0.5, 3, 0)
+        return lib.dasha_m3d_write_ctx(d.h, path, 0.5)
+
+    assert out() == capi.OK
+    good = {p.name: p.read_bytes() for p in tmp_path.iterdir()}
+    d.stepon(0.0, d.setdt(0.0), 0)
+    assert lib.dasha_check_ring_wait(d.h) == capi.OK
+    assert out() == capi.E_CUDA
+    assert {p.name: p.read_bytes() for p in tmp_path.iterdir()} == good
+    d.close()
