@@ -719,7 +719,7 @@ int dasha_timer(dasha_ctx* c, int op, double* ms) {
     float f = 0.f;
     if (cudaEventElapsedTime(&f, e->t0, e->t1) != cudaSuccess) return fail(c, DASHA_E_CUDA, "cudaEventElapsedTime failed");
     *ms = f;
-    return DASHA_OK;
+    return wait_status(c, DASHA_OK);
 }
 
 int dasha_profile(dasha_ctx* c, int enable) {
@@ -751,7 +751,7 @@ int dasha_profile_read(dasha_ctx* c, int* n, char* names, double* ms, long* laun
     *n = (int)nt;
     p.recs.clear();
     p.used = 0;
-    return DASHA_OK;
+    return wait_status(c, DASHA_OK);
 }
 
 // ---- z-slab groups (halo.h) ----

@@ -46,12 +46,13 @@ def test_contexts_stepped_in_turn_keep_apart(precisions):
 
 
 @pytest.mark.parametrize("precision", [0, 1], ids=["fp64", "fp32"])
-@pytest.mark.parametrize("call", ["setdt", "get_state", "diagnostics"])
+@pytest.mark.parametrize("call", ["setdt", "get_state", "diagnostics", "timer_stop", "profile_read"])
 def test_a_ring_wait_is_reported_by_its_own_context(call, precision):
     lib = capi.bind(capi.BOUNDS_LIB_PATH)
     lib.dasha_check_ring_wait.argtypes = [C.c_void_p]
     a, b = (capi.gem_context(CFGS[0], precision, lib=lib) for _ in range(2))
     dt = a.setdt(0.0)
+    a.timer_start()
     a.stepon(0.0, dt, 0)
     assert lib.dasha_check_ring_wait(a.h) == capi.OK
     b.stepon(0.0, b.setdt(0.0), 0)
