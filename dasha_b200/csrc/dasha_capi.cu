@@ -146,8 +146,8 @@ static int wait_status(dasha_ctx*, int rc) { return rc; }
 #endif
 
 // `waits`: wait for the stream and look for ring waits that ran out.  dasha_stepon, which only enqueues, and dasha_setdt,
-// whose own copy brings the answer, do without on a whole-grid context: two waits with an idle GPU after each, 43 us
-// of a 661 us step on 64x32x64 FP64.
+// whose own copy brings the answer, do without on a whole-grid context, periodic or bounded: two waits with an idle GPU
+// after each, 43 us of a 661 us step on 64x32x64 FP64.
 template <class F>
 static int host_call(dasha_ctx* c, F body, bool waits = true) {
     try {

@@ -67,6 +67,9 @@ public:
     long n = 0;
     bool eq_set = false;
 
+    // no kernel here waits on a ring: stepon enqueues, and setdt waits for its own copy
+    bool own_wait_status() const override { return true; }
+
     ~WallEngine() override {
         if (pool) cudaFree(pool);
         if (tab) cudaFree(tab);
