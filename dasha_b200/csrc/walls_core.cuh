@@ -398,8 +398,13 @@ struct RowRule {
 
 // A loop over the physical nodes that gives every field its values after a boundary routine: out(m, c,
 // value) with c the node's index.  The nodes behind the x-min rows take a thread for all NF fields, or one
-// per field (split) where the grid is too small to fill the GPU so: 41x25x33 takes 0.84 ms a step
-// split and 0.95 ms not, 129x72x101 6.2 and 4.6 ms.  Those of the x-min rows, three smoothed values each, come after
+// per field (split) on small grids.  Split threads are shorter, but do what the fields share NF times, so they
+// win while they all run at once.  Loops of 3 fields turn a little above one wave of eight blocks of 128 an SM (the threads of
+// the boundary rows are short): ms a step with their loops split / not, 52896 nodes 0.681 / 0.748, 54180 0.721 / 0.736, 58800
+// 0.855 / 0.781, 60000 0.936 / 0.809.  Loops of 8 fields, which share more of the work, turn at the same
+// size (52896 0.733 / 0.748, 58800 0.771 / 0.781, 60000 0.828 / 0.809, 64000 0.792 / 0.771), so one line serves
+// both: 9/8 of a wave of 3-field threads.  All loops: 9600 nodes 0.549 / 0.648, 33825 0.632 / 0.745,
+// 84150 0.964 / 0.849, 464520 3.63 / 2.87, 997458 7.41 / 5.79.  Those of the x-min rows, three smoothed values each, come after
 // them with a thread per field, so that no warp holds both (10.3 ms a step with them in line).
 template <int NF, class S, class Out>
 struct RowLoop {
@@ -494,7 +499,7 @@ struct Core {
     }
     template <int NF, class S, class Out>
     void rows(const S& s, const RowRule& rr, const Out& out) {
-        const bool split = (long)d.mx * d.my * d.mz < 100000;   // below a thread for each of 148 SMs' slots, about
+        const bool split = 3L * d.mx * d.my * d.mz <= 148L * 9 * 128;
         ex.run({1, ((d.mx - 2) * (split ? NF : 1) + 2 * NF) * d.my * d.mz, 1, 1, 1, 1}, RowLoop<NF, S, Out>{s, rr, out, split});
     }
 
