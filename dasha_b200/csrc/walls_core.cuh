@@ -29,6 +29,8 @@
 #include <cmath>
 #include <vector>
 
+#include "quotient.h"
+
 #if !defined(__CUDACC__)
 #define __host__
 #define __device__
@@ -82,25 +84,16 @@ struct Arr {
 WHD inline double d1fc(double fm2, double fm, double f0, double fp, double fp2, double a, double b, double c, double d) {
     return a * (fp - f0) + b * (f0 - fm) + c * (fp2 - f0) + d * (f0 - fm2);
 }
-// a / b rounded to nearest, r the reciprocal 1 / b rounded to nearest.  On the device by two
-// remainder corrections with fused multiply-adds (Markstein, IBM J. Res. Dev. 34, 1990: with r = RN(1/b)
-// and a quotient q off by at most an ulp, q + r RN(a - q b) is RN(a / b); the first correction makes q such):
-// five operations instead of the division's branch and some thirty.  Quotients that could overflow or be
-// subnormal in between, zeros, infinities and NaN take the division.  Checked against the division
-// bit for bit in the smoothing passes (the bounded engine equals the loops that divide).
+// a / b rounded to nearest, r the reciprocal 1 / b rounded to nearest: on the device by two remainder corrections, five
+// operations instead of the division's branch and some thirty.  Quotients that could overflow or be subnormal in between, zeros,
+// infinities and NaN take the division.
 WHD inline double div_by(double a, double b, double r) {
 #ifdef __CUDA_ARCH__
-    // the exponents of a and r within 2^+-650 and 2^+-300
-    const unsigned ea = ((unsigned)__double2hiint(a) >> 20) & 0x7ffu, er = ((unsigned)__double2hiint(r) >> 20) & 0x7ffu;
-    if (ea - 373u < 1300u && er - 723u < 600u) {
-        double q = a * r;
-        q = __fma_rn(__fma_rn(-q, b, a), r, q);
-        return __fma_rn(__fma_rn(-q, b, a), r, q);
-    }
+    return div_by_steps(a, b, r);
 #else
     (void)r;
-#endif
     return a / b;
+#endif
 }
 // one direction of the smoothing difference: hp, hm the spacings x+ - x0, x0 - x-, h2 = x+ - x-, r2 = 1 / h2
 WHD inline double difc(double fm, double f0, double fp, double hp, double hm, double h2, double r2) {

@@ -36,6 +36,7 @@
 
 #include <type_traits>
 
+#include "quotient.h"
 #include "tma.cuh"
 
 namespace dasha {
@@ -74,6 +75,7 @@ __device__ __forceinline__ void l2_fetch(const void* p) { asm volatile("prefetch
 // were slower. ----
 template <class T, int NF, int VX>
 struct VStore {
+    static constexpr int MIN_CTAS = 0;             // no bound
     T* f[NF];
     struct Pre {};
     __device__ __forceinline__ void pre(long, Pre&) const {}
@@ -105,26 +107,18 @@ struct VSum {
     }
 };
 
-// a / d for d = 3 or 6, r = RN(1 / d), rounded to nearest: a r is within an ulp of the quotient (RN(1/3) is off by
-// a third of an ulp), so one remainder correction gives it (Markstein, IBM J. Res. Dev. 34, 1990); where that
-// correction is undefined (an infinite a) the product stands.  Below 2^-100 (FP32) or 2^-960 (FP64) the remainder may
-// itself round.  Four operations and a select instead of the division's thirty and its branch, for the RK update's two quotients
-// a node and field: 277 -> 244 us (256x128x256 FP64, stage 2), 39 -> 29.5 us (128x60x90 FP64), 515 -> 458 us
-// (512x256x256 FP32), the same bits in every run compared.
-template <class T>
-__device__ __forceinline__ T over(T a, T d, T r) {
-    const T q = a * r;
-    T e;
-    if constexpr (sizeof(T) == 4) e = __fmaf_rn(__fmaf_rn(-q, d, a), r, q);
-    else e = __fma_rn(__fma_rn(-q, d, a), r, q);
-    return e == e ? e : q;
-}
-
+// The quotients by 3 and 6 a node and field take over() (quotient.h), some eight operations instead of the division's thirty
+// and its branch: 277 -> 244 us (256x128x256 FP64, stage 2), 39 -> 29.5 us (128x60x90 FP64), 515 -> 458 us
+// (512x256x256 FP32), 4 fields.  Of that, the division's bits for subnormal sixths and zeros cost 1-6 % of a launch (both groups of
+// fields, 256x128x256 FP64 404 -> 422, 463 -> 464, 471 -> 478, 389 -> 415 us in stages 1-4) and nothing of a step.
+//
 // RK4 stage update with the smoothed xdif (stepon t3dsdsc.f:1090-1132): plain registers
 // (base, acc = xm, x) in FP64; in FP32 acc holds only the increment and the base update of
 // stage 4 is a Kahan step with the compensation comp (value = x - comp).
 template <class T, int NF, int VX, bool KAHAN>
 struct VRK {
+    // FP64: the registers that leave 3 CTAs an SM (the compiler's own choice, 186, leaves 2)
+    static constexpr int MIN_CTAS = sizeof(T) == 8 ? 3 : 0;
     T* x[NF];
     const T* base[NF];
     T* acc[NF];
@@ -193,6 +187,7 @@ struct VRK {
 // the result set to the exact halves / zeros of rows 2 and mz-3 (bndrytt)
 template <class T, int NF, int VX>
 struct VKF {
+    static constexpr int MIN_CTAS = 0;             // no bound
     T* x[NF];
     T* comp[NF];
     struct Pre { T x[NF][VX], k[NF][VX]; };
@@ -594,7 +589,7 @@ __global__ void __launch_bounds__(32 * TYH) k_zpv_two(Geo<T> g, SrcFields<T, NF>
 
 #ifndef DASHA_NO_TMA
 template <class T, int NF, unsigned KA, unsigned KB, int VX, int TYH, int RY, int D, class EA, class EB, int MODE = 0>
-__global__ void __launch_bounds__(32 * TYH) k_zpv_two_tma(Geo<T> g, SrcFields<T, NF> sa, EA ea, SrcFields<T, NF> sb, EB eb,
+__global__ void __launch_bounds__(32 * TYH, EA::MIN_CTAS) k_zpv_two_tma(Geo<T> g, SrcFields<T, NF> sa, EA ea, SrcFields<T, NF> sb, EB eb,
                                                           int chunk, int nz, const __grid_constant__ ZpMaps ma,
                                                           const __grid_constant__ ZpMaps mb) {
     if ((int)blockIdx.z < nz) zpv_body<T, NF, KA, VX, TYH, RY, D, EA, MODE, true>(g, sa, ea, chunk, (int)blockIdx.z, &ma);
