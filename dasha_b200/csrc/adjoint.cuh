@@ -507,20 +507,4 @@ static __global__ void k_adj_psi(Geo<double> g, const double* sbx, const double*
                                     b[p1] * g.b1x[p1] + b[i2] * g.c1x[i2] - b[p2] * g.d1x[p2];
 }
 
-// forward psi map: dBx = -Dz psi (interior rows), dBz = Dx psi, added to the state
-static __global__ void k_psi_apply(Geo<double> g, const double* psi, double* bx, double* bz, double s) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= g.mx) return;
-    int j = blockIdx.y, k = blockIdx.z;
-    long c = (long)i + (long)j * g.sy + (long)k * g.sz;
-    const double* P = psi;
-    auto ps = [&](int ii, int kk) { return P[(long)wrapi(ii, g.mx) + (long)kk * g.mx]; };
-    double dz = 0.0;
-    if (k >= 2 && k <= g.mz - 3)
-        dz = d1fc(ps(i, k - 2), ps(i, k - 1), ps(i, k), ps(i, k + 1), ps(i, k + 2), g.a1z[k], g.b1z[k], g.c1z[k], g.d1z[k]);
-    double dx = d1fc(ps(i - 2, k), ps(i - 1, k), ps(i, k), ps(i + 1, k), ps(i + 2, k), g.a1x[i], g.b1x[i], g.c1x[i], g.d1x[i]);
-    bx[c] += s * (-dz);
-    bz[c] += s * dx;
-}
-
 }  // namespace dasha

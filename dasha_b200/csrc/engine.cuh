@@ -623,7 +623,6 @@ public:
     static F3<T> f3(T* const* p) { F3<T> r; for (int m = 0; m < 3; ++m) r.f[m] = p[m]; return r; }
 
     // ---- z-marching launches ----
-    static constexpr int TX = 32, TY = 8;
     // CTAs per SM of a kernel, asked once per context (a member: several builds of the library may
     // share a process, and a function-local static of a template would be shared between them)
     std::vector<std::pair<const void*, int>> resident_of;
@@ -892,7 +891,6 @@ public:
     }
     static constexpr int HMINB = sizeof(T) == 4 ? 2 : 1;   // CTAs per SM asked of the register allocator
     static SrcFields<T, 3> src3(T* const* p) { SrcFields<T, 3> s; for (int q = 0; q < 3; ++q) s.f[q] = p[q]; return s; }
-    static SrcFields<T, 8> src8(T* const* p) { SrcFields<T, 8> s; for (int q = 0; q < 8; ++q) s.f[q] = p[q]; return s; }
     static St3 st3(T* const* p) { St3 s; for (int q = 0; q < 3; ++q) s.f[q] = p[q]; return s; }
     static constexpr unsigned KIND_H = 1u | (1u << 2) | (1u << 4);                 // 1/8 for 3 fields
     static constexpr unsigned KIND_B4 = 2u | (2u << 2) | (2u << 4);                 // fields 4..7: B1 B2 B3 p
@@ -1164,7 +1162,7 @@ public:
         }
         if (nstep % 10 == 0) {      // diagn blow-up guard (t3dsdsc.f:1174-1182, 1232)
             hx(X + 4, 3);           // the current reads B at z-neighbours
-            Status s = launch_diag(true);
+            Status s = launch_diag();
             if (s.code) return s;
         }
         DASHA_CK(cudaGetLastError());
@@ -1176,13 +1174,12 @@ public:
         return Status::ok();
     }
 
-    Status launch_diag(bool guard_only) {
+    Status launch_diag() {
         launch_current(X);
         double* rows = red;
         double* fl = red + 2L * my * mz;
         double* jext = fl + my;
         double* out = red + nred;
-        (void)guard_only;
         // the planes this context accounts for and its planes of the central z plane(s): all of
         // them on a whole grid; on a z-slab its own planes (and the walls it holds), and the
         // flux where it owns the (first) central plane, the second one an own or ghost plane
@@ -1207,7 +1204,7 @@ public:
 
     Status diagnostics(double* outh) override {
         hx(X + 4, 3);   // a z-slab: the current and a central plane may read B's ghost planes
-        Status s = launch_diag(false);
+        Status s = launch_diag();
         if (s.code) return s;
         DASHA_CK(cudaMemcpyAsync(hpin, red + nred, sizeof(double) * DASHA_NDIAG, cudaMemcpyDeviceToHost, st));
         DASHA_CK(cudaStreamSynchronize(st));
@@ -1319,7 +1316,6 @@ public:
     static size_t adj_field_bytes(long n) { return ((size_t)n * sizeof(double) + 255) & ~(size_t)255; }
     struct V8 { T* f[8]; };
 
-    void k8(T** d, T* const* s2) { for (int m = 0; m < 8; ++m) d[m] = s2[m]; }
     void copy8(T* const* dst, T* const* src) {
         DASHA_LAUNCH("a_copy8", 16.0 * N * sizeof(T),
                      for (int m = 0; m < 8; ++m) cudaMemcpyAsync(dst[m], src[m], sizeof(T) * N, cudaMemcpyDeviceToDevice, st));
