@@ -201,10 +201,12 @@ public:
     double* red = nullptr;       // reduction scratch
     double* cfltab = nullptr;    // CFL rate tables: ich[mx+my+mz], vv[..], ih[..]
     // bits of setdt's largest rate, two words taken in turn (a sweep clears the other one), then the
-    // blow-up flag, then whether a ring wait of this context ran out (g.late): one copy reads all
+    // blow-up flag, then whether a ring wait of this context ran out (late): one copy reads all
     unsigned long long* rate_bits = nullptr;
     int rate_word = 0;
     int* flag = nullptr;         // blow-up flag
+    unsigned* late = nullptr;    // a ring wait ran out (set by the TMA kernels, through their maps: Geo, which every kernel
+                                 // takes, is left as small as it is)
     double* hpin = nullptr;      // pinned host scratch
     double* mpd = nullptr;       // the 11 mid-plane output fields (allocated on first use)
     Geo<T> g{};
@@ -226,7 +228,7 @@ public:
     }
     void set_cfl_k0(int k0) override { g.kcfl0 = k0; }
     bool own_wait_status() const override { return !halo; }
-    unsigned* ring_late() override { return g.late; }
+    unsigned* ring_late() override { return late; }
     // a z-slab with a neighbour: its ghost planes are copies (a lone slab's are the walls)
     bool cut() const { return halo && (halo->geo.lower() || halo->geo.upper()); }
     // z-slab contexts: refresh the ghost planes of fields f that a later launch reads at
@@ -360,7 +362,7 @@ public:
         DASHA_CK(cudaMalloc(&rate_bits, 32));
         DASHA_CK(cudaMemsetAsync(rate_bits, 0, 32, st));
         flag = (int*)(rate_bits + 2);
-        g.late = (unsigned*)(rate_bits + 3);
+        late = (unsigned*)(rate_bits + 3);
         DASHA_CK(cudaMallocHost(&hpin, sizeof(double) * 16));
 
         blk = dim3(std::min(128, ((mx + 31) / 32) * 32));
@@ -676,6 +678,7 @@ public:
     template <int NF>
     bool zpv_maps(const SrcFields<T, NF>& src, ZpMaps& m) {
         using Z = ZVc<NF>;
+        m.late = late;
         EncodeTiledFn enc = encode_tiled();
         if (!enc) return false;
         const cuuint64_t dims[3] = {(cuuint64_t)mx, (cuuint64_t)my, (cuuint64_t)mz};
@@ -831,7 +834,7 @@ public:
     // FP64 512x256x512, ms a step: 8 rows, 1 CTA 16.6; 4 rows, 3 CTAs 12.8.
     static constexpr int ZH_TY = 4, ZH_MINB = sizeof(T) == 4 ? 4 : 3;
     static constexpr int ZHP_TY = 6, ZHP_MINB = 2;
-    // Pairs halve the instructions per node (522 -> 332), but a plane's step is longer and its tile larger, so they
+    // Pairs save a quarter of the instructions per node (442 -> 319 on 512x256x128), but a plane's step is longer and its tile larger, so they
     // lose where few tiles leave each CTA its latency (one node against pairs, us: 64x32x64 12.9 / 14.9, 6 tiles a
     // plane; 100x44x77 21.0 / 21.1, 16; 128x64x96 27.7 / 27.1, 22; 128x128x64 35.4 / 33.3, 44) and where the tiles hang over
     // the grid (32x200x50, half of each tile unused, 18.3 / 23.0; the gain at full tiles is about 1/7).  The rule is
@@ -973,11 +976,13 @@ public:
         return (n & 1) ? b : a;
     }
     // The Hall chain's passes 1-4 as two fused pairs (k_zpv2), or one by one with the E chain's passes (k_zpv_two)?  Pairs save
-    // a read and a write of the fields, passes the halo and level-1 work of 320-thread CTAs: on large planes, where memory
-    // sets the pace, pairs win (1024x512x512 FP32 181.2 against 182.7 ms a step), on 512x256 planes and below the
-    // passes do (512x256x256 FP32 22.64 against 22.85, 512x256x512 FP64 86.4 against 88.0, 64x32x64 FP32 0.289
-    // against 0.339); FP64, whose passes are longer, at every size measured.  Both give the same values: a pair rounds as
-    // two single passes.  A z-slab takes the passes: k_zpv2 forms its first pass next to the slab ends from the wall rule.
+    // a read and a write of the fields, passes the halo and level-1 work of 320-thread CTAs.  FP32, ms a step, passes against
+    // pairs: 64x32x64 0.289 / 0.339, 512x256x256 22.56 / 22.73, 768x320x96 16.1 / 16.2, 768x384x96 19.32 / 19.40, 512x256x512
+    // 44.8 / 44.6, 768x384x256 50.26 / 50.19, 1024x512x96 33.57 / 33.61, 768x512x256 67.04 / 66.85, 1024x384x256 66.56 / 66.42,
+    // 1024x512x256 88.44 / 87.95, 1024x512x512 182.7 / 181.2: passes lead on small grids, pairs by up to 0.8 % on large ones, and
+    // from 300 thousand to 400 thousand nodes a plane the two are within 0.4 %, so that the line between them is of little weight.
+    // It is on the plane, which a grid of any depth shares.  FP64, whose passes are longer, takes passes at every size
+    // (512x256x512 86.4 / 88.0).  Both give the same values: a pair rounds as two single passes.  A z-slab takes the passes: k_zpv2 forms its first pass next to the slab ends from the wall rule.
     bool hall_pairs() const { return KAHAN && !cut() && (long)mx * my > 262144; }
 
     // smoothed current of state xs (current, t3dsdsc.f:2452-2500): curl, 4 passes
@@ -986,6 +991,7 @@ public:
     // the five ring fields of k_zhydro as tensor maps, boxes of one ring plane (RS x NR x 1)
     template <class Z>
     bool hydro_maps(const HydroIO<T>& io, ZhMaps& m) {
+        m.late = late;
         EncodeTiledFn enc = encode_tiled();
         if (!enc) return false;
         const T* f[5] = {io.m1, io.m2, io.m3, io.dp, io.drho};
@@ -1236,9 +1242,9 @@ public:
         DASHA_CK(cudaGetLastError());
         DASHA_CK(cudaMemcpyAsync(hpin + 12, rate_bits, 32, cudaMemcpyDeviceToHost, st));
         DASHA_CK(cudaStreamSynchronize(st));
-        unsigned late = 0;
-        std::memcpy(&late, hpin + 15, sizeof(late));
-        if (late) return Status::err(DASHA_E_CUDA, RING_WAIT_MSG);
+        unsigned ran_out = 0;
+        std::memcpy(&ran_out, hpin + 15, sizeof(ran_out));
+        if (ran_out) return Status::err(DASHA_E_CUDA, RING_WAIT_MSG);
         const double v = hpin[12 + word];
         *dt = (v != v) ? v : std::fmin(100.0, 1.0 / v);
         std::memcpy(blowup, hpin + 14, sizeof(int));

@@ -29,7 +29,6 @@ struct Geo {
     // difc weights: difc = (f+ - f0)*wp - (f0 - f-)*wm  (t3dsdsc.f:5618-5619)
     const T *wpx, *wmx, *wpy, *wmy, *wpz, *wmz;
     const T *cbx;    // (1/32)(1 - tanh((x+3)/8)), smoothing coefficient of B (t3dsdsc.f:5636-5642)
-    unsigned* late;  // set by a launch of the context whose bounded ring wait ran out
     const T* cr;     // FP64 contexts: the radial coefficient below at every node, made once (k_radial_field)
     const T *xc, *yc, *zc;   // node coordinates: the radial coefficient 1/32 + 3/32 (1 + tanh((r-3)/3))/2
                              // (t3dsdsc.f:5659-5661); FP32 passes evaluate it per node
@@ -182,8 +181,8 @@ __device__ __forceinline__ double warp_sum(double v) {
 // CFL in rate form: the reference's per-direction step h / (vp/cfl + visc/(2h)) is the
 // inverse of the rate vp * (1/(cfl h)) + visc/(2 h^2), so dt = min(100, 1 / max rate) over
 // the region k 0..mz-3, j 0..my-2, i 0..mx-3 (t3dsdsc.f:4709-4736).  Tables per axis:
-// ich = 1/(cfl |h|), vv = visc/(2 h^2), ih = 1/|h| (whistler term).  One block per (j,k)
-// row; NaN wins so that a corrupted state is reported.
+// ich = 1/(cfl |h|), vv = visc/(2 h^2), ih = 1/|h| (whistler term).  NaN wins so that a corrupted
+// state is reported.
 __device__ __forceinline__ double nanmax(double a, double b) { return (a != a || b != b) ? (a != a ? a : b) : fmax(a, b); }
 
 // The CFL rate of node c (totals = equilibrium profile at the node's plane + stored

@@ -1,6 +1,6 @@
 // tma.cuh -- ring planes of the z-marching kernels loaded by `cp.async.bulk.tensor` against one
-// mbarrier per ring stage, with waits that give up after about a second (recorded in Geo::late, the context's
-// own word, and reported by its next call that waits) instead of spinning.  Built unless -DDASHA_NO_TMA (the comparison build
+// mbarrier per ring stage, with waits that give up after about a second (recorded in a word of the context
+// itself, and reported by its next call that waits) instead of spinning.  Built unless -DDASHA_NO_TMA (the comparison build
 // whose rings all use cp.async).
 #pragma once
 

@@ -3,10 +3,10 @@
 // equation, for the case without viscosity and diffusion; z-marching and register-blocked.
 //
 // A warp covers 32*VX consecutive x nodes, one row per warp, TY warps per CTA.  FP32 grids of some
-// size take VX = 2: issue slots bound the kernel (63 % used by one node per thread at 522 instructions a
-// node, where memory needs 333 of 779 us on 512x256x256), and a thread that owns two nodes loads float
+// size take VX = 2: issue slots bound the kernel (57 % used by one node per thread at 442 instructions a
+// node on 512x256x128; memory needs 333 of 779 us on 512x256x256), and a thread that owns two nodes loads float
 // pairs, forms and differences its fluxes as packed pairs with no register moves, and shares the tile's halo of
-// 1/rho among more nodes: 332 instructions a node, 779 -> 645 us.  Planes of m1, m2, m3, p - p0 and rho - rho0 (tile plus a 2-node x/y halo, no
+// 1/rho among more nodes: 319 instructions a node, 779 -> 645 us.  Planes of m1, m2, m3, p - p0 and rho - rho0 (tile plus a 2-node x/y halo, no
 // corners) stream into an NS = D + 5 stage shared-memory ring with cp.async; the thread whose
 // copy landed turns rho - rho0 into 1/rho in place.  The five quantities of the own nodes for
 // planes c-2 .. c+2 stay in a register queue (the z stencil), so per plane a thread reads plane
@@ -21,7 +21,7 @@
 // rows y0-2 .. y0+TY+1) lies inside the grid loads each ring plane as 5 `cp.async.bulk.tensor`
 // boxes of exactly the ring plane's layout, issued by thread 0 against one mbarrier per stage;
 // every thread waits on the stage's mbarrier (time-bounded: after about a second the kernel
-// sets Geo::late, waits, again bounded, for the boxes it issued and returns) and turns
+// sets the context's word, waits, again bounded, for the boxes it issued and returns) and turns
 // its share of the plane's rho - rho0 into 1/rho before the plane's barrier.  CTAs whose halo
 // wraps around x or y keep the cp.async element copies (a box cannot wrap).  The compute is the
 // same code in both kernels; the engine picks one.
@@ -34,7 +34,10 @@
 namespace dasha {
 
 // the five ring fields (m1 m2 m3 dp drho) as 3-D tensor maps with the box of one ring plane
-struct ZhMaps { CUtensorMap m[5]; };
+struct ZhMaps {
+    CUtensorMap m[5];
+    unsigned* late;                                   // as in ZpMaps
+};
 
 template <class T, int VX, int TY, int D>
 struct ZH {
@@ -223,7 +226,7 @@ __device__ __forceinline__ void zhydro_body(const Geo<T>& g, const HydroIO<T>& i
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             if (__syncthreads_or(late)) {
                 // every box issued so far (planes up to c+2+D) lands before the CTA leaves
-                if (tid == 0) atomicExch(g.late, 1u);
+                if (tid == 0) atomicExch(maps->late, 1u);
                 for (int p = c - 2; p <= min(c + 2 + D, phi); ++p) {
                     if (p < cA - 2) continue;
                     mbar_wait_bounded(bars + p % NS, (unsigned)(((p - (cA - 2)) / NS) & 1));

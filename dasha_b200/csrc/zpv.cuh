@@ -11,16 +11,15 @@
 // instead of 5.  Only planes c and c+1 are read in a plane step, so the stage refilled at step c
 // (plane c+1+D, the stage of plane c-2) is neither of the two planes still read by threads in
 // step c-1: one barrier per plane suffices; the first step also reads plane c-1 and so ends with
-// a second barrier.  (Loading the planes by TMA instead, as ring-plane boxes with one mbarrier
-// per stage, measured 7-40 % slower per pass on B200 in every arrangement tried: the passes are
-// issue-bound and cp.async's per-thread copies cost about 2 % of their instructions.)
+// a second barrier.
 //
 // TMA (k_zpv_tma; not built with -DDASHA_NO_TMA): a CTA whose ring box (x0-OFF .. x0+TX+OFF-1, rows
 // y0-1 .. y0+TY) lies inside the grid loads each ring plane as NF `cp.async.bulk.tensor` boxes of
 // exactly the ring plane's layout, issued by thread 0 against one mbarrier per stage; every thread
 // waits (time-bounded) on the stages it reads before the plane's barrier.  CTAs whose halo wraps
 // keep the cp.async copies.  The compute is the same code in both kernels; the engine picks one
-// per launch.
+// per launch: TMA in FP64 (4-9 % faster) and for the FP32 passes of 4 and 6 fields, cp.async for the FP32 passes of 3, whose
+// 3 CTAs of 8 warps overlap the per-thread copies with their arithmetic (TMA 10 % slower).
 //
 // KINDS: 2 bits per output field, 0 radial coefficient, 1 constant 1/8, 2 x-profile cbx.  The
 // radial coefficient is evaluated per node in FP32 (__expf) and read from the context's field
@@ -41,8 +40,12 @@
 
 namespace dasha {
 
-// the source fields of a pass as 3-D tensor maps with the box of one ring plane (k_zpv_tma)
-struct ZpMaps { CUtensorMap m[8]; };
+// the source fields of a pass as 3-D tensor maps with the box of one ring plane (k_zpv_tma), and the context's word for
+// ring waits that ran out
+struct ZpMaps {
+    CUtensorMap m[8];
+    unsigned* late;
+};
 
 // VX consecutive values of a field, one access (8-byte aligned float pairs in FP32)
 template <class T, int VX>
@@ -381,7 +384,7 @@ __device__ __forceinline__ void zpv_body(const Geo<T>& g, const SrcFields<T, NF>
                 if (!mbar_wait_bounded(bars + p % NS, (unsigned)(((p - (cA - 1)) / NS) & 1))) { late = true; break; }
             if (__syncthreads_or(late)) {
                 // every box issued so far (planes up to c+1+D) lands before the CTA leaves
-                if (tid == 0) atomicExch(g.late, 1u);
+                if (tid == 0) atomicExch(maps->late, 1u);
                 for (int p = c - 1; p <= min(c + 1 + D, phi); ++p)
                     if (p >= cA - 1) mbar_wait_bounded(bars + p % NS, (unsigned)(((p - (cA - 1)) / NS) & 1));
                 return;
