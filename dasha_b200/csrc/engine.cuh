@@ -725,7 +725,7 @@ public:
 #ifndef DASHA_NO_TMA
         if constexpr (zp_tma<NF>()) {
             ZpMaps maps;
-            if (!zpv_maps<NF>(src, maps)) launch_err = "cuTensorMapEncodeTiled failed for a smoothing pass";
+            if (!zpv_maps<NF>(src, maps)) { launch_err = "cuTensorMapEncodeTiled failed for a smoothing pass"; return; }
             DASHA_LAUNCH(tag, bytes, launch(zpv_tma_fn<NF, KINDS, Epi, MODE>(), gg, 32 * ZC<NF>::TYH, Z::smem_tma(), g, src, epi, ch, maps));
         } else
 #endif
@@ -795,7 +795,7 @@ public:
             const int ch = zchunk(tiles, (const void*)fn, 32 * ZC<NF>::TYH, Z::smem_tma()), nz = (mz + ch - 1) / ch;
             gg.z = 2 * nz;
             ZpMaps ma, mb;
-            if (!zpv_maps<NF>(sa, ma) || !zpv_maps<NF>(sb, mb)) launch_err = "cuTensorMapEncodeTiled failed for a smoothing pass";
+            if (!zpv_maps<NF>(sa, ma) || !zpv_maps<NF>(sb, mb)) { launch_err = "cuTensorMapEncodeTiled failed for a smoothing pass"; return; }
             DASHA_LAUNCH(tag, bytes, launch(fn, gg, 32 * ZC<NF>::TYH, Z::smem_tma(), g, sa, ea, sb, eb, ch, nz, ma, mb));
         } else
 #endif
@@ -1020,7 +1020,7 @@ public:
         gh.z = (mz + chh - 1) / chh;
 #ifndef DASHA_NO_TMA
         ZhMaps maps;
-        if (!hydro_maps<Z>(hio, maps)) launch_err = "cuTensorMapEncodeTiled failed for the hydro ring";
+        if (!hydro_maps<Z>(hio, maps)) { launch_err = "cuTensorMapEncodeTiled failed for the hydro ring"; return; }
         DASHA_LAUNCH("k_rhs_hydro", 16.0 * N * sizeof(T),
                      launch(k_zhydro_tma<T, VX, TY, 1, MINB>, gh, 32 * TY, Z::smem_tma(), g, hio, chh, maps));
 #else
@@ -1171,9 +1171,13 @@ public:
             Status s = launch_diag();
             if (s.code) return s;
         }
+        return launched();
+    }
+
+    // the launches so far: a CUDA error, or one that could not be set up and was left out
+    Status launched() {
         DASHA_CK(cudaGetLastError());
-        if (launch_err) {
-            const char* e = launch_err;
+        if (const char* e = launch_err) {
             launch_err = nullptr;
             return Status::err(DASHA_E_CUDA, e);
         }
@@ -1214,11 +1218,8 @@ public:
         if (s.code) return s;
         DASHA_CK(cudaMemcpyAsync(hpin, red + nred, sizeof(double) * DASHA_NDIAG, cudaMemcpyDeviceToHost, st));
         DASHA_CK(cudaStreamSynchronize(st));
-        if (launch_err) {
-            const char* e = launch_err;
-            launch_err = nullptr;
-            return Status::err(DASHA_E_CUDA, e);
-        }
+        s = launched();
+        if (s.code) return s;
         for (int q = 0; q < DASHA_NDIAG; ++q) outh[q] = hpin[q];
         int none = 0;
         if (halo && halo->per_process() && !halo->reduce_diag(outh, &none))
@@ -1261,12 +1262,7 @@ public:
     Status current(double* curh, long ld1, long ld2) override {
         hx(X + 4, 3);
         launch_current(X);
-        DASHA_CK(cudaGetLastError());
-        if (launch_err) {
-            const char* e = launch_err;
-            launch_err = nullptr;
-            return Status::err(DASHA_E_CUDA, e);
-        }
+        if (Status s = launched(); s.code) return s;
         return transfer_out(curh, ld1, ld2, curF, 3, false);
     }
 
@@ -1279,7 +1275,7 @@ public:
         F8<T> cz;
         for (int m = 0; m < 8; ++m) cz.f[m] = KAHAN ? C[m] : nullptr;
         launch(k_midplane<T>, dim3((mx + 127) / 128, mz), 128, 0, g, my / 2, f8(X), cz, f3(curF), mpd);
-        DASHA_CK(cudaGetLastError());
+        if (Status s = launched(); s.code) return s;
         DASHA_CK(cudaMemcpyAsync(outh, mpd, sizeof(double) * 11 * (size_t)mx * mz, cudaMemcpyDeviceToHost, st));
         DASHA_CK(cudaStreamSynchronize(st));
         return Status::ok();
@@ -1287,7 +1283,7 @@ public:
 
     Status current_out(const ChunkOut& take) override {
         launch_current(X);
-        DASHA_CK(cudaGetLastError());
+        if (Status s = launched(); s.code) return s;
         return stream_out(curF, 3, false, nullptr, take);
     }
 
@@ -1295,12 +1291,11 @@ public:
         T* out[8];
         for (int m = 0; m < 8; ++m) out[m] = S[m];
         launch_rhs(X, t != 0.0, out);
-        DASHA_CK(cudaGetLastError());
+        if (Status s = launched(); s.code) return s;
         return transfer_out(xdif, ld1, ld2, out, 8, false);
     }
 
     // ======================= discrete adjoint (FP64 contexts) =======================
-    // scratch of one adjoint call (cudaMalloc'd per call, freed at the end)
     // scratch of one adjoint call: one cudaMalloc carved into fields (freed at the end)
     struct AdjBufs {
         char* base = nullptr;
@@ -1320,7 +1315,6 @@ public:
         ~AdjBufs() { if (base) cudaFree(base); }
     };
     static size_t adj_field_bytes(long n) { return ((size_t)n * sizeof(double) + 255) & ~(size_t)255; }
-    struct V8 { T* f[8]; };
 
     void copy8(T* const* dst, T* const* src) {
         DASHA_LAUNCH("a_copy8", 16.0 * N * sizeof(T),
@@ -1468,7 +1462,7 @@ public:
             Status s2 = transfer_in(wh, ld1, ld2, kap, 8, false);
             if (s2.code) return s2;
             adj_rhs(X, kap, sig, w);
-            DASHA_CK(cudaGetLastError());
+            if (Status s3 = launched(); s3.code) return s3;
             return transfer_out(outh, ld1, ld2, sig, 8, false);
         }
     }
@@ -1589,7 +1583,7 @@ public:
             if (!dpsi_d) return Status::err(DASHA_E_NOMEM, "adjoint scratch");
             k_adj_ysum<<<dim3((mx + blk.x - 1) / blk.x, mz, 1), blk, 0, st>>>(g, v.lam[4], v.lam[6], w.jt[0], w.jt[1]);
             k_adj_psi<<<dim3((mx + blk.x - 1) / blk.x, mz, 1), blk, 0, st>>>(g, w.jt[0], w.jt[1], dpsi_d);
-            DASHA_CK(cudaGetLastError());
+            if (Status s3 = launched(); s3.code) return s3;
             std::vector<double> hp((size_t)mx * mz);
             DASHA_CK(cudaMemcpyAsync(hp.data(), dpsi_d, sizeof(double) * mx * mz, cudaMemcpyDeviceToHost, st));
             double he = 0.0;
