@@ -139,6 +139,20 @@ public:
         }
         return Status::ok();
     }
+    // the rows [0, n) of a chunk, by the calling thread alone in a transfer of at most `alone` bytes, by the host threads above.
+    // To wake the threads takes some 20 us, and rows on their way up leave the cache of the thread that the caller
+    // filled them on, from which the copy to the GPU then reads slower.  Median ms a call, threads / alone (the padded copy
+    // before), set_state: 10x10x10 0.103 / 0.062 (0.043), 41x25x33 (2.2 MB) 0.55 / 0.30 (0.40), 49x30x40 0.84 / 0.50 (0.66),
+    // 74x45x59 (12.6 MB) 1.6-2.0 / 0.88-1.0 (2.0), 98x60x79 (30 MB) 2.6-3.1 / 2.0-2.2 (5.0), 115x70x92 (47 MB) 3.8 / 3.2 (10),
+    // 200x120x150 (230 MB) 17.6 / 17.5 (71); get_state: 10x10x10 0.077 / 0.048 (0.055), 41x25x33 0.39-0.41 / 0.36-0.42 (0.41),
+    // 49x30x40 0.57-0.63 / 0.58-0.65 (0.66), 55x34x45 (5.4 MB) 0.74-0.98 / 0.50-0.59 (0.9), 66x40x53 (9 MB) 1.0-1.6 / 0.8-1.0 (1.4),
+    // 74x45x59 0.98-1.7 / 0.95-1.2 (1.9), 98x60x79 1.1-3.0 / 2.2-2.7 (4.4), 200x120x150 15.3 / 25.4 (45).
+    static constexpr size_t ALONE_UP = size_t(32) << 20, ALONE_DOWN = size_t(10) << 20;
+    template <class F>
+    void spread(long rows, size_t alone, long n, const F& f) const {
+        if (sizeof(double) * (size_t)rows * d.mx <= alone) f(0L, n);
+        else HostPool::get().run(n, f);
+    }
     // host address of row r = j + my (k + mz m) of the caller's array
     long row_at(long r, long ld1, long ld2) const {
         const long j = r % d.my, q = r / d.my, k = q % d.mz, m = q / d.mz;
@@ -153,7 +167,7 @@ public:
             const long r1 = std::min(rows, r0 + step);
             double* h = pin[q & 1];
             DASHA_CK(cudaEventSynchronize(pev[q & 1]));
-            HostPool::get().run(r1 - r0, [&](long a0, long a1) {
+            spread(rows, ALONE_UP, r1 - r0, [&](long a0, long a1) {
                 for (long r = a0; r < a1; ++r) std::memcpy(h + r * d.mx, src + row_at(r0 + r, ld1, ld2), sizeof(double) * d.mx);
             });
             DASHA_CK(cudaMemcpyAsync(stage + r0 * d.mx, h, sizeof(double) * (size_t)(r1 - r0) * d.mx, cudaMemcpyHostToDevice, st));
@@ -182,7 +196,7 @@ public:
             DASHA_CK(cudaEventSynchronize(pev[q & 1]));
             const long r0 = q * step, r1 = std::min(rows, r0 + step);
             const double* h = pin[q & 1];
-            HostPool::get().run(r1 - r0, [&](long a0, long a1) {
+            spread(rows, ALONE_DOWN, r1 - r0, [&](long a0, long a1) {
                 for (long r = a0; r < a1; ++r) std::memcpy(dst + row_at(r0 + r, ld1, ld2), h + r * d.mx, sizeof(double) * d.mx);
             });
         }

@@ -50,3 +50,22 @@ def test_calls_behind_enqueued_steps(grid):
     assert np.array_equal(a.get_state(), b.get_state())
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("grid", [(5, 7, 9), (41, 25, 33), (66, 40, 53), (129, 72, 101)], ids=lambda g: "x".join(map(str, g)))
+def test_states_come_back_as_they_went(grid):
+    """both ways of gathering the rows, one and several chunks, pageable and pinned: the state of dasha_get_state is that of
+    dasha_set_state, and the caller's halo stays as it was"""
+    from dasha_b200 import harris
+    d, X = _context(grid)
+    rng = np.random.default_rng(2)
+    for _ in range(2):
+        Y = X * (1 + 0.1 * rng.standard_normal(X.shape))
+        d.set_state(Y)
+        H = harris.to_halo(np.zeros_like(X))
+        H[:] = 7.0
+        assert d.lib.dasha_get_state(d.h, capi._dp(H), H.shape[3], H.shape[2]) == capi.OK
+        assert np.array_equal(harris.from_halo(H, *grid), Y)
+        H[:, 2:-2, :, 2:-2] = 7.0
+        assert (H == 7.0).all()
+    d.close()
