@@ -125,7 +125,11 @@ public:
     cudaEvent_t pev[2] = {nullptr, nullptr};
     std::vector<double> small_buf;
     static constexpr size_t PIN = size_t(8) << 20, SMALL = size_t(4) << 20;
-    long chunk_rows() const { return std::max(1L, (long)(PIN / sizeof(double)) / d.mx); }
+    // rows of one pinned buffer: two of them hold an 8-field array of up to 16 MB (to pin memory takes about 1 ms a MB)
+    long chunk_rows() const {
+        const long most = std::max(1L, (long)(PIN / sizeof(double)) / d.mx);
+        return small_buf.empty() ? std::min(most, 4L * d.my * d.mz) : most;
+    }
     Status pins() {
         if (pev[1]) return Status::ok();
         const size_t all = 8 * sizeof(double) * (size_t)d.mx * d.my * d.mz;
